@@ -166,11 +166,12 @@ typedef struct lbm_lattice {
  *     (warps 1..8 per CTA).
  *   pipeline LBM_PIPE_SPLIT: the register/shuffle pull over static work lists of row
  *     segments (lbm_build_worklists): plain interior segments run a lean kernel that reads
- *     no flag words, edge segments the same plus the x-edge copies and inlet/outlet
- *     extrapolation, special segments (walls, bed, lid, banks, hulls, forcing) a separately
- *     compiled general one, and solid segments move no populations (cells_per_lane 2 or 4
+ *     no flag words, edge segments a similar one with the x-edge copies and inlet/outlet
+ *     extrapolation, special segments (walls, bed, banks, hulls, forcing) a general one with
+ *     one cell per lane, and solid segments move no populations (cells_per_lane 2 or 4
  *     as the lists were built; warps 1..4 per CTA).
- * ctas_per_sm: resident CTAs per SM of the persistent grid (0 = as many as fit). */
+ * ctas_per_sm: resident CTAs per SM of a persistent grid; 0 = as many as fit, and for the split
+ *   pipeline's lists one warp pass per warp (CTAs come and go in list order). */
 #define LBM_PIPE_REGISTER 0
 #define LBM_PIPE_TMA 1
 #define LBM_PIPE_ASYNC 2
@@ -242,11 +243,10 @@ int lbm_unpack_populations(const lbm_lattice *lat, const uint16_t *h, float *f, 
 /* One fused time step hs -> hd on 16-bit storage; same physics, modes and fields as
  * lbm_fused_step.  Requires pitch % 8 == 0, work lists built with cells_per_lane 2, 4 or 8 (row
  * segments of 64, 128 or 256 cells) and tile {LBM_PIPE_SPLIT, that cells_per_lane, warps 1..4,
- * stages, ctas_per_sm} (NULL tile = 2 cells per lane, 4 warps, as many CTAs per SM as fit).
- * Plain segments move `stages` = 8 (or 0) cells per lane with 16-byte accesses, or 4 cells per
- * lane with 8-byte accesses (stages = 4, lists of 64 or 128 cells); edge and special segments
- * run the general path with 2 cells per lane (cells_per_lane 2) or 4 (one pass, or two for
- * 256-cell segments). */
+ * stages, ctas_per_sm} (NULL tile = 2 cells per lane, 4 warps, one pass per warp).
+ * Plain segments move `stages` = 4 (or 0) cells per lane with 8-byte accesses (lists of 64 or 128
+ * cells), or 8 cells per lane with 16-byte accesses (stages = 8, and always on 256-cell segments);
+ * edge segments move four cells per lane, special segments one. */
 int lbm_fused_step_h(const lbm_lattice *lat, const uint16_t *hs, uint16_t *hd, float scale, uint32_t mode,
                      const lbm_tile *tile, void *stream);
 
@@ -279,7 +279,7 @@ int lbm_batch_pull_offsets_bytes(void);
 int lbm_batch_init(const lbm_batch *b, void *stream);
 
 /* One step of every lattice of the batch; mode = LBM_STEP_* bits (for all lattices); tile
- * {LBM_PIPE_SPLIT, 2, warps 1..4, stages (plain-kernel cells per lane 8, or 4; 0 = 8),
+ * {LBM_PIPE_SPLIT, 2, warps 1..4, stages (plain-kernel cells per lane 4, or 8; 0 = 4),
  * ctas_per_sm}, NULL = {LBM_PIPE_SPLIT, 2, 4, 0, 0}. */
 int lbm_batch_step_h(const lbm_batch *b, int parity, uint32_t mode, const lbm_tile *tile, void *stream);
 

@@ -19,9 +19,9 @@ from . import _native as nat
 # kernels beside the plain kernel (LBM3D.overlap), ctas_per_sm then bounding the plain kernel.
 SINGLE_FP32 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 4), (3, 4, 2, 0, 0), (0, 2, 4, 0, 0),
                (3, 4, 4, 0, 0, 1), (3, 4, 4, 0, 2, 1), (3, 2, 4, 0, 2, 1)]
-SINGLE_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 4, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 2), (3, 8, 4, 0, 0),
+SINGLE_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 8, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 2), (3, 8, 4, 0, 0),
                (3, 2, 4, 0, 0, 1), (3, 2, 4, 0, 2, 1), (3, 2, 4, 0, 1, 1)]
-BATCH_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 4, 0), (3, 2, 4, 0, 2), (3, 2, 1, 0, 0)]
+BATCH_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 8, 0), (3, 2, 4, 0, 2), (3, 2, 1, 0, 0)]
 
 _memo: dict = {}
 

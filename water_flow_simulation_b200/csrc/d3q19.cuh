@@ -4,6 +4,7 @@
 // (floodsim/lbm3d.py:16-21); they are constexpr functions so that, inside fully
 // unrolled direction loops, every c_i, w_i and index folds to a literal.
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 namespace wfs {
@@ -43,13 +44,39 @@ constexpr uint32_t FLAG_WALLFN = 1u << 21;     // wall function applies (cf > 0 
 constexpr uint32_t FLAG_BEDWALL = 1u << 22;    // bed/bank wall cell: reference speed is the column mean
 constexpr uint32_t FLAG_GHOST = 1u << 23;      // x padding beyond nx (treated as solid)
 
-// A float product rounded on its own (never fused into a later add).
+// Float operations with their rounding fixed: a product or sum rounded on its own, a
+// multiply-add rounded once.  The collision and the inlet/outlet rule are written in these, so
+// that every kernel that inlines them computes the same bits whatever the compiler would fuse.
 __host__ __device__ __forceinline__ float mul_rn(float a, float b)
 {
 #ifdef __CUDA_ARCH__
     return __fmul_rn(a, b);
 #else
     return a * b;
+#endif
+}
+__host__ __device__ __forceinline__ float add_rn(float a, float b)
+{
+#ifdef __CUDA_ARCH__
+    return __fadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+__host__ __device__ __forceinline__ float sub_rn(float a, float b)
+{
+#ifdef __CUDA_ARCH__
+    return __fsub_rn(a, b);
+#else
+    return a - b;
+#endif
+}
+__host__ __device__ __forceinline__ float fma_rn(float a, float b, float c)
+{
+#ifdef __CUDA_ARCH__
+    return __fmaf_rn(a, b, c);
+#else
+    return fmaf(a, b, c);
 #endif
 }
 
@@ -63,6 +90,9 @@ __host__ __device__ __forceinline__ float mul_rn(float a, float b)
 //   C  = 4.5 [ rho u u + (1-om) Pi + sf (u F + F u) ]      (sf = 1 - om/2)
 // which needs no per-direction equilibrium.  On return f holds the post-collision
 // populations and r/ux/uy/uz the cell's density and velocity.
+// FORCED false: no body force (the terms in F drop out).
+// UX2: round ux^2 on its own in |u|^2 (kernels that also accumulate ux^2 share the product), else uy^2.
+template <bool FORCED, bool UX2 = false>
 __host__ __device__ __forceinline__ void collide(float (&f)[Q], float fx, float fy, float fz, float tau0, float csmag2,
                                         float& r, float& ux, float& uy, float& uz)
 {
@@ -85,45 +115,64 @@ __host__ __device__ __forceinline__ void collide(float (&f)[Q], float fx, float 
     const float sxy = s7 - s9, sxz = s11 - s13, syz = s15 - s17;
 
     const float ir = 1.0f / r;
-    ux = (jx + 0.5f * fx) * ir;
-    uy = (jy + 0.5f * fy) * ir;
-    uz = (jz + 0.5f * fz) * ir;
-    const float r3 = r * (1.0f / 3.0f);
-    const float pxx = sxx - r * ux * ux - r3, pyy = syy - r * uy * uy - r3, pzz = szz - r * uz * uz - r3;
-    const float pxy = sxy - r * ux * uy, pxz = sxz - r * ux * uz, pyz = syz - r * uy * uz;
+    ux = mul_rn(FORCED ? fma_rn(0.5f, fx, jx) : jx, ir);
+    uy = mul_rn(FORCED ? fma_rn(0.5f, fy, jy) : jy, ir);
+    uz = mul_rn(FORCED ? fma_rn(0.5f, fz, jz) : jz, ir);
+    // the products r u u serve both the stress and the equilibrium
+    const float rx = mul_rn(r, ux), ry = mul_rn(r, uy), rz = mul_rn(r, uz);
+    const float rxx = mul_rn(rx, ux), ryy = mul_rn(ry, uy), rzz = mul_rn(rz, uz);
+    const float rxy = mul_rn(rx, uy), rxz = mul_rn(rx, uz), ryz = mul_rn(ry, uz);
+    const float third = -(1.0f / 3.0f);
+    const float pxx = fma_rn(third, r, sub_rn(sxx, rxx)), pyy = fma_rn(third, r, sub_rn(syy, ryy)),
+                pzz = fma_rn(third, r, sub_rn(szz, rzz));
+    const float pxy = sub_rn(sxy, rxy), pxz = sub_rn(sxz, rxz), pyz = sub_rn(syz, ryz);
 
-    const float qn = sqrtf(pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * (pxy * pxy + pxz * pxz + pyz * pyz));
-    // tau0^2 and 18 sqrt(2) Cs^2 are rounded explicitly: they are lattice constants, and a compiler
-    // that hoists them out of a loop (or not) must not change how they fuse into what follows
+    const float qd = fma_rn(pzz, pzz, fma_rn(pxx, pxx, mul_rn(pyy, pyy)));
+    const float qo = fma_rn(pyz, pyz, fma_rn(pxy, pxy, mul_rn(pxz, pxz)));
+    const float qn = sqrtf(fma_rn(2.0f, qo, qd));
     const float tau0sq = mul_rn(tau0, tau0), smag = mul_rn(18.0f * 1.41421356f, csmag2);
-    const float tau = 0.5f * (tau0 + sqrtf(tau0sq + smag * qn * ir));
+    const float tau = mul_rn(0.5f, add_rn(tau0, sqrtf(fma_rn(mul_rn(smag, qn), ir, tau0sq))));
     const float om = 1.0f / tau;
-    const float k1 = 1.0f - om, sf = 1.0f - 0.5f * om;
+    const float k1 = sub_rn(1.0f, om);
 
-    const float usq = ux * ux + uy * uy + uz * uz;
-    const float uF = ux * fx + uy * fy + uz * fz;
-    const float A0 = r - 1.5f * (r * usq + k1 * (pxx + pyy + pzz)) - 3.0f * sf * uF;
-    const float bf = 3.0f * sf - 1.5f * k1;
-    const float Bx = 3.0f * r * ux + bf * fx, By = 3.0f * r * uy + bf * fy, Bz = 3.0f * r * uz + bf * fz;
-    const float Cxx = 4.5f * (r * ux * ux + k1 * pxx + 2.0f * sf * ux * fx);
-    const float Cyy = 4.5f * (r * uy * uy + k1 * pyy + 2.0f * sf * uy * fy);
-    const float Czz = 4.5f * (r * uz * uz + k1 * pzz + 2.0f * sf * uz * fz);
-    const float Cxy2 = 9.0f * (r * ux * uy + k1 * pxy + sf * (ux * fy + fx * uy));
-    const float Cxz2 = 9.0f * (r * ux * uz + k1 * pxz + sf * (ux * fz + fx * uz));
-    const float Cyz2 = 9.0f * (r * uy * uz + k1 * pyz + sf * (uy * fz + fy * uz));
-
+    const float usq = fma_rn(uz, uz, UX2 ? fma_rn(uy, uy, mul_rn(ux, ux)) : fma_rn(ux, ux, mul_rn(uy, uy)));
+    const float trace = add_rn(add_rn(pxx, pyy), pzz);
+    float A0 = fma_rn(-1.5f, fma_rn(k1, trace, mul_rn(r, usq)), r);
+    const float r3 = mul_rn(3.0f, r);
+    float Bx = mul_rn(r3, ux), By = mul_rn(r3, uy), Bz = mul_rn(r3, uz);
+    float Cxx = fma_rn(k1, pxx, rxx), Cyy = fma_rn(k1, pyy, ryy), Czz = fma_rn(k1, pzz, rzz);
+    float Cxy = fma_rn(k1, pxy, rxy), Cxz = fma_rn(k1, pxz, rxz), Cyz = fma_rn(k1, pyz, ryz);
+    if constexpr (FORCED) {
+        const float sf = fma_rn(-0.5f, om, 1.0f);
+        const float uF = fma_rn(uz, fz, fma_rn(uy, fy, mul_rn(ux, fx)));
+        A0 = fma_rn(mul_rn(-3.0f, sf), uF, A0);
+        const float bf = fma_rn(-1.5f, k1, mul_rn(3.0f, sf));
+        Bx = fma_rn(bf, fx, Bx);
+        By = fma_rn(bf, fy, By);
+        Bz = fma_rn(bf, fz, Bz);
+        const float sf2 = mul_rn(2.0f, sf);
+        Cxx = fma_rn(mul_rn(sf2, ux), fx, Cxx);
+        Cyy = fma_rn(mul_rn(sf2, uy), fy, Cyy);
+        Czz = fma_rn(mul_rn(sf2, uz), fz, Czz);
+        Cxy = fma_rn(sf, fma_rn(fx, uy, mul_rn(ux, fy)), Cxy);
+        Cxz = fma_rn(sf, fma_rn(fx, uz, mul_rn(ux, fz)), Cxz);
+        Cyz = fma_rn(sf, fma_rn(fy, uz, mul_rn(uy, fz)), Cyz);
+    }
+    // f_i = w_i (A0 + c.B + c.C.c), C's factors 4.5 (diagonal) and 9 (off-diagonal) applied here
     constexpr float w0 = wgt(0), w1 = wgt(1), w2 = wgt(7);
-    f[0] = w0 * A0;
-    float b;
-    b = A0 + Cxx;                 f[1] = w1 * (b + Bx);  f[2] = w1 * (b - Bx);
-    b = A0 + Cyy;                 f[3] = w1 * (b + By);  f[4] = w1 * (b - By);
-    b = A0 + Czz;                 f[5] = w1 * (b + Bz);  f[6] = w1 * (b - Bz);
-    b = A0 + Cxx + Cyy + Cxy2;    f[7] = w2 * (b + (Bx + By));  f[8] = w2 * (b - (Bx + By));
-    b = A0 + Cxx + Cyy - Cxy2;    f[9] = w2 * (b + (Bx - By));  f[10] = w2 * (b - (Bx - By));
-    b = A0 + Cxx + Czz + Cxz2;    f[11] = w2 * (b + (Bx + Bz)); f[12] = w2 * (b - (Bx + Bz));
-    b = A0 + Cxx + Czz - Cxz2;    f[13] = w2 * (b + (Bx - Bz)); f[14] = w2 * (b - (Bx - Bz));
-    b = A0 + Cyy + Czz + Cyz2;    f[15] = w2 * (b + (By + Bz)); f[16] = w2 * (b - (By + Bz));
-    b = A0 + Cyy + Czz - Cyz2;    f[17] = w2 * (b + (By - Bz)); f[18] = w2 * (b - (By - Bz));
+    f[0] = mul_rn(w0, A0);
+    const float bx = fma_rn(4.5f, Cxx, A0), by = fma_rn(4.5f, Cyy, A0), bz = fma_rn(4.5f, Czz, A0);
+    f[1] = mul_rn(w1, add_rn(bx, Bx));  f[2] = mul_rn(w1, sub_rn(bx, Bx));
+    f[3] = mul_rn(w1, add_rn(by, By));  f[4] = mul_rn(w1, sub_rn(by, By));
+    f[5] = mul_rn(w1, add_rn(bz, Bz));  f[6] = mul_rn(w1, sub_rn(bz, Bz));
+    const float bxy = fma_rn(4.5f, Cyy, bx), bxz = fma_rn(4.5f, Czz, bx), byz = fma_rn(4.5f, Czz, by);
+    float b, B;
+    b = fma_rn(9.0f, Cxy, bxy);   B = add_rn(Bx, By);  f[7] = mul_rn(w2, add_rn(b, B));  f[8] = mul_rn(w2, sub_rn(b, B));
+    b = fma_rn(-9.0f, Cxy, bxy);  B = sub_rn(Bx, By);  f[9] = mul_rn(w2, add_rn(b, B));  f[10] = mul_rn(w2, sub_rn(b, B));
+    b = fma_rn(9.0f, Cxz, bxz);   B = add_rn(Bx, Bz);  f[11] = mul_rn(w2, add_rn(b, B)); f[12] = mul_rn(w2, sub_rn(b, B));
+    b = fma_rn(-9.0f, Cxz, bxz);  B = sub_rn(Bx, Bz);  f[13] = mul_rn(w2, add_rn(b, B)); f[14] = mul_rn(w2, sub_rn(b, B));
+    b = fma_rn(9.0f, Cyz, byz);   B = add_rn(By, Bz);  f[15] = mul_rn(w2, add_rn(b, B)); f[16] = mul_rn(w2, sub_rn(b, B));
+    b = fma_rn(-9.0f, Cyz, byz);  B = sub_rn(By, Bz);  f[17] = mul_rn(w2, add_rn(b, B)); f[18] = mul_rn(w2, sub_rn(b, B));
 }
 
 // Direction masks over bits 1..18 (bit i = direction i), for popcount sums over a wall mask.
@@ -141,6 +190,52 @@ __host__ __device__ __forceinline__ int popc32(uint32_t v)
     return __popc(v);
 #else
     return __builtin_popcount(v);
+#endif
+}
+
+// The wall function's small-integer float64 operations, exact or correctly rounded like the
+// general ones they stand for, without the conversion unit's or the square root's latency:
+// int_double -- a small signed integer: its bits under the exponent of 2^52, less the bias;
+// sqrt_small -- the square root of 0..12, tabulated;
+// div_small  -- p / n for n = 1..75 by Markstein's correction (IBM J. Res. Dev. 34, 1990): with y the
+//               correctly rounded 1/n and q0 = p y, q0 + (p - q0 n) y rounds to the quotient.
+#ifdef __CUDACC__
+constexpr int kSmallDivisors = 76;
+struct SmallTables {
+    double root[13], inverse[kSmallDivisors];
+};
+constexpr SmallTables small_tables()
+{
+    SmallTables t{{0.0, 1.0, 1.4142135623730951, 1.7320508075688772, 2.0, 2.23606797749979, 2.449489742783178, 2.6457513110645907, 2.8284271247461903, 3.0, 3.1622776601683795, 3.3166247903554, 3.4641016151377544},
+                  {}};
+    for (int k = 1; k < kSmallDivisors; ++k) t.inverse[k] = 1.0 / k;
+    return t;
+}
+__device__ __constant__ constexpr SmallTables kSmall = small_tables();
+#endif
+__host__ __device__ __forceinline__ double int_double(int k)
+{
+#ifdef __CUDA_ARCH__
+    return __hiloint2double(0x43300000, k ^ (int)0x80000000) - 4503601774854144.0;       // 2^52 + 2^31
+#else
+    return k;
+#endif
+}
+__host__ __device__ __forceinline__ double sqrt_small(int k)
+{
+#ifdef __CUDA_ARCH__
+    return kSmall.root[k];
+#else
+    return sqrt((double)k);
+#endif
+}
+__host__ __device__ __forceinline__ double div_small(double p, int n)
+{
+#ifdef __CUDA_ARCH__
+    const double y = kSmall.inverse[n], d = int_double(n), q = p * y;
+    return fma(fma(-q, d, p), y, q);
+#else
+    return p / n;
 #endif
 }
 
@@ -193,10 +288,11 @@ __host__ __device__ __forceinline__ void wall_function(float (&f)[Q], uint32_t w
     //   s = us0/ut = (-2 (t.J) - rw cf U^2 area ut) / (6 rw t^T M t)
     // the update is f_i += w_i c_i.(6 rw clamp(s, -1, 1) t): one square root for ut, one for
     // the face area, one division -- the same quantities as the reference's, regrouped.
-    const double area = sqrt((double)a2);
-    const double pn = (double)px * nwx + (double)py * nwy + (double)pz * nwz;
-    const double q = pn / (double)n2;
-    const double tx = px - q * nwx, ty = py - q * nwy, tz = pz - q * nwz;
+    const double area = sqrt_small(a2);
+    const double nx = int_double(nwx), ny = int_double(nwy), nz = int_double(nwz);
+    const double pn = (double)px * nx + (double)py * ny + (double)pz * nz;
+    const double q = div_small(pn, n2);
+    const double tx = px - q * nx, ty = py - q * ny, tz = pz - q * nz;
     const double ut = sqrt(tx * tx + ty * ty + tz * tz);
     if (!(ut > 1e-7)) return;
     double jx = 0.0, jy = 0.0, jz = 0.0;
@@ -210,12 +306,12 @@ __host__ __device__ __forceinline__ void wall_function(float (&f)[Q], uint32_t w
         }
     const double tJ = tx * jx + ty * jy + tz * jz;
     const double w1 = (double)wgt(1), w2 = (double)wgt(7);
-    const double mxx = w1 * popc32(wx & AXIS) + w2 * popc32(wx & ~AXIS);
-    const double myy = w1 * popc32(wy & AXIS) + w2 * popc32(wy & ~AXIS);
-    const double mzz = w1 * popc32(wz & AXIS) + w2 * popc32(wz & ~AXIS);
-    const double mxy = w2 * (popc32(wm & XY_SAME) - popc32(wm & XY_OPP));
-    const double mxz = w2 * (popc32(wm & XZ_SAME) - popc32(wm & XZ_OPP));
-    const double myz = w2 * (popc32(wm & YZ_SAME) - popc32(wm & YZ_OPP));
+    const double mxx = w1 * int_double(popc32(wx & AXIS)) + w2 * int_double(popc32(wx & ~AXIS));
+    const double myy = w1 * int_double(popc32(wy & AXIS)) + w2 * int_double(popc32(wy & ~AXIS));
+    const double mzz = w1 * int_double(popc32(wz & AXIS)) + w2 * int_double(popc32(wz & ~AXIS));
+    const double mxy = w2 * int_double(popc32(wm & XY_SAME) - popc32(wm & XY_OPP));
+    const double mxz = w2 * int_double(popc32(wm & XZ_SAME) - popc32(wm & XZ_OPP));
+    const double myz = w2 * int_double(popc32(wm & YZ_SAME) - popc32(wm & YZ_OPP));
     const double tMt = tx * tx * mxx + ty * ty * myy + tz * tz * mzz + 2.0 * (tx * ty * mxy + tx * tz * mxz + ty * tz * myz);
     if (!(tMt > 0.0)) return;
     const double U = uref > 0.f ? (double)uref : ut;
@@ -245,9 +341,8 @@ __host__ __device__ __forceinline__ void wall_function(float (&f)[Q], uint32_t w
 //   B = 3 (rho_b u_b - rho_g u_g),  C = 4.5 (rho_b u_b u_b - rho_g u_g u_g),
 // so it is evaluated like the collision's output stage (one pass, no per-direction
 // equilibria); the result differs from the reference's order of operations only by
-// float32 rounding.
-template <bool INLET>
-__host__ __device__ __forceinline__ void nebb(const float (&g)[Q], float (&out)[Q], float uin, float rho_out)
+// float32 rounding.  `inlet` is a runtime switch, so that one copy of the code serves both ends.
+__host__ __device__ __forceinline__ void nebb(bool inlet, const float (&g)[Q], float (&out)[Q], float uin, float rho_out)
 {
     const float s1 = g[1] + g[2], d1 = g[1] - g[2];
     const float s3 = g[3] + g[4], d3 = g[3] - g[4];
@@ -263,31 +358,40 @@ __host__ __device__ __forceinline__ void nebb(const float (&g)[Q], float (&out)[
     const float my = d3 + d7 - d9 + d15 + d17;
     const float mz = d5 + d11 - d13 + d15 - d17;
     const float ir = 1.0f / r;
-    const float ux = mx * ir, uy = my * ir, uz = mz * ir;
-    // rho_b u_b and rho_b u_b u_b minus the same of g
-    float rb, bx, by, bz;
-    if (INLET) { rb = r; bx = uin; by = 0.f; bz = 0.f; }
-    else       { rb = rho_out; bx = ux; by = uy; bz = uz; }
-    const float A = (rb - r) - 1.5f * (rb * (bx * bx + by * by + bz * bz) - r * (ux * ux + uy * uy + uz * uz));
-    const float Bx = 3.0f * (rb * bx - r * ux), By = 3.0f * (rb * by - r * uy), Bz = 3.0f * (rb * bz - r * uz);
-    const float Cxx = 4.5f * (rb * bx * bx - r * ux * ux);
-    const float Cyy = 4.5f * (rb * by * by - r * uy * uy);
-    const float Czz = 4.5f * (rb * bz * bz - r * uz * uz);
-    const float Cxy2 = 9.0f * (rb * bx * by - r * ux * uy);
-    const float Cxz2 = 9.0f * (rb * bx * bz - r * ux * uz);
-    const float Cyz2 = 9.0f * (rb * by * bz - r * uy * uz);
+    const float ux = mul_rn(mx, ir), uy = mul_rn(my, ir), uz = mul_rn(mz, ir);
+    const float rb = inlet ? r : rho_out, bx = inlet ? uin : ux, by = inlet ? 0.f : uy, bz = inlet ? 0.f : uz;
+    const float usq = fma_rn(uz, uz, fma_rn(ux, ux, mul_rn(uy, uy)));
+    const float bsq = fma_rn(bz, bz, fma_rn(bx, bx, mul_rn(by, by)));
+    const float A = fma_rn(-1.5f, fma_rn(rb, bsq, -mul_rn(r, usq)), sub_rn(rb, r));
+    // rho u and rho u u of the boundary state less those of g
+    const float rx = mul_rn(r, ux), ry = mul_rn(r, uy), rz = mul_rn(r, uz);
+    const float px = mul_rn(rb, bx), py = mul_rn(rb, by), pz = mul_rn(rb, bz);
+    const float jx = sub_rn(px, rx), jy = sub_rn(py, ry), jz = sub_rn(pz, rz);
+    const float Bx = mul_rn(3.0f, jx), By = mul_rn(3.0f, jy), Bz = mul_rn(3.0f, jz);
+    const float Cxx = fma_rn(px, bx, -mul_rn(rx, ux)), Cyy = fma_rn(py, by, -mul_rn(ry, uy)),
+                Czz = fma_rn(pz, bz, -mul_rn(rz, uz));
+    const float Cxy = fma_rn(px, by, -mul_rn(rx, uy)), Cxz = fma_rn(px, bz, -mul_rn(rx, uz)),
+                Cyz = fma_rn(py, bz, -mul_rn(ry, uz));
     constexpr float w0 = wgt(0), w1 = wgt(1), w2 = wgt(7);
-    out[0] = g[0] + w0 * A;
-    float b;
-    b = A + Cxx;                 out[1] = g[1] + w1 * (b + Bx);  out[2] = g[2] + w1 * (b - Bx);
-    b = A + Cyy;                 out[3] = g[3] + w1 * (b + By);  out[4] = g[4] + w1 * (b - By);
-    b = A + Czz;                 out[5] = g[5] + w1 * (b + Bz);  out[6] = g[6] + w1 * (b - Bz);
-    b = A + Cxx + Cyy + Cxy2;    out[7] = g[7] + w2 * (b + (Bx + By));  out[8] = g[8] + w2 * (b - (Bx + By));
-    b = A + Cxx + Cyy - Cxy2;    out[9] = g[9] + w2 * (b + (Bx - By));  out[10] = g[10] + w2 * (b - (Bx - By));
-    b = A + Cxx + Czz + Cxz2;    out[11] = g[11] + w2 * (b + (Bx + Bz)); out[12] = g[12] + w2 * (b - (Bx + Bz));
-    b = A + Cxx + Czz - Cxz2;    out[13] = g[13] + w2 * (b + (Bx - Bz)); out[14] = g[14] + w2 * (b - (Bx - Bz));
-    b = A + Cyy + Czz + Cyz2;    out[15] = g[15] + w2 * (b + (By + Bz)); out[16] = g[16] + w2 * (b - (By + Bz));
-    b = A + Cyy + Czz - Cyz2;    out[17] = g[17] + w2 * (b + (By - Bz)); out[18] = g[18] + w2 * (b - (By - Bz));
+    out[0] = fma_rn(w0, A, g[0]);
+    const float bxx = fma_rn(4.5f, Cxx, A), byy = fma_rn(4.5f, Cyy, A), bzz = fma_rn(4.5f, Czz, A);
+    out[1] = fma_rn(w1, fma_rn(3.0f, jx, bxx), g[1]);  out[2] = fma_rn(w1, fma_rn(-3.0f, jx, bxx), g[2]);
+    out[3] = fma_rn(w1, fma_rn(3.0f, jy, byy), g[3]);  out[4] = fma_rn(w1, fma_rn(-3.0f, jy, byy), g[4]);
+    out[5] = fma_rn(w1, fma_rn(3.0f, jz, bzz), g[5]);  out[6] = fma_rn(w1, fma_rn(-3.0f, jz, bzz), g[6]);
+    const float bxy = fma_rn(4.5f, Cyy, bxx), bxz = fma_rn(4.5f, Czz, bxx), byz = fma_rn(4.5f, Czz, byy);
+    float b, c;
+    b = fma_rn(9.0f, Cxy, bxy);   c = fma_rn(3.0f, jx, By);
+    out[7] = fma_rn(w2, add_rn(b, c), g[7]);   out[8] = fma_rn(w2, sub_rn(b, c), g[8]);
+    b = fma_rn(-9.0f, Cxy, bxy);  c = fma_rn(3.0f, jx, -By);
+    out[9] = fma_rn(w2, add_rn(b, c), g[9]);   out[10] = fma_rn(w2, sub_rn(b, c), g[10]);
+    b = fma_rn(9.0f, Cxz, bxz);   c = fma_rn(3.0f, jx, Bz);
+    out[11] = fma_rn(w2, add_rn(b, c), g[11]); out[12] = fma_rn(w2, sub_rn(b, c), g[12]);
+    b = fma_rn(-9.0f, Cxz, bxz);  c = fma_rn(3.0f, jx, -Bz);
+    out[13] = fma_rn(w2, add_rn(b, c), g[13]); out[14] = fma_rn(w2, sub_rn(b, c), g[14]);
+    b = fma_rn(9.0f, Cyz, byz);   c = add_rn(By, Bz);
+    out[15] = fma_rn(w2, add_rn(b, c), g[15]); out[16] = fma_rn(w2, sub_rn(b, c), g[16]);
+    b = fma_rn(-9.0f, Cyz, byz);  c = sub_rn(By, Bz);
+    out[17] = fma_rn(w2, add_rn(b, c), g[17]); out[18] = fma_rn(w2, sub_rn(b, c), g[18]);
 }
 
 }  // namespace wfs

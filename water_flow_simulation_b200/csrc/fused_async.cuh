@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256, 2) k_fused_async(const lbm_lattice L, con
             const bool fast = rwm == 0 && !edge_seg && __all_sync(0xffffffffu, (fk & kSpecial) == 0);
             if (fast) {
                 read_all_interior(std::make_integer_sequence<int, Q>{}, f, slot + xi + 4);
-                collide(f, 0.f, 0.f, 0.f, L.tau0, L.csmag2, R, UX, UY, UZ);
+                collide<false>(f, 0.f, 0.f, 0.f, L.tau0, L.csmag2, R, UX, UY, UZ);
             } else if (fk & FLAG_SOLID) {
                 R = 1.f; UX = 0.f; UY = 0.f; UZ = 0.f;
 #pragma unroll
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(256, 2) k_fused_async(const lbm_lattice L, con
                     fy = L.Fy[c] * L.force_scale;
                     fz = L.Fz[c] * L.force_scale;
                 }
-                collide(f, fx, fy, fz, L.tau0, L.csmag2, R, UX, UY, UZ);
+                collide<true>(f, fx, fy, fz, L.tau0, L.csmag2, R, UX, UY, UZ);
             }
             // inlet: x=0 (lane 0 of the first group of segment 0) from x=1 (lane 1)
             if (x0 == 0 && k == 0) {
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256, 2) k_fused_async(const lbm_lattice L, con
                 for (int i = 0; i < Q; ++i) g[i] = __shfl_down_sync(0xffffffffu, f[i], 1);
                 const uint32_t f1 = __shfl_down_sync(0xffffffffu, fk, 1);
                 if (lane == 0 && !(fk & FLAG_SOLID) && !(f1 & FLAG_SOLID))
-                    nebb<true>(g, f, L.uin[y + (long long)L.ny * z], L.rho_out);
+                    nebb(true, g, f, L.uin[y + (long long)L.ny * z], L.rho_out);
             }
             // outlet: x=nx-1 from x=nx-2, one lane lower in the same 32-cell group
             if (outlet_fused && x0 + 32 * k <= L.nx - 1 && L.nx - 1 < x0 + 32 * k + 32) {
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256, 2) k_fused_async(const lbm_lattice L, con
 #pragma unroll
                 for (int i = 0; i < Q; ++i) g[i] = __shfl_up_sync(0xffffffffu, f[i], 1);
                 const uint32_t fm = __shfl_up_sync(0xffffffffu, fk, 1);
-                if (x == L.nx - 1 && !(fk & FLAG_SOLID) && !(fm & FLAG_SOLID)) nebb<false>(g, f, 0.f, L.rho_out);
+                if (x == L.nx - 1 && !(fk & FLAG_SOLID) && !(fm & FLAG_SOLID)) nebb(false, g, f, 0.f, L.rho_out);
             }
 #pragma unroll
             for (int i = 0; i < Q; ++i) outb[i * kSegA + xi] = f[i];

@@ -5,8 +5,8 @@
 // descriptors, pull-offset tables, 16-bit storage scales and both population buffers of each.
 // Work-list entries carry the case in their top 8 bits and the row-segment id (of that case's
 // own 64-cell segments, cells_per_lane 2) in the low 24.  One step of the whole batch is then
-// a plain, an edge and a general launch over the concatenated lists (plus the solid-field,
-// column-mean and outlet passes on output steps), whatever the sizes of the cases: small
+// a plain launch and one for the special and edge cells over the concatenated lists (plus the
+// solid-field, column-mean and outlet passes on output steps), whatever the sizes of the cases: small
 // cases no longer leave the GPU idle between launches or in short tails, and the launch
 // count of a step does not grow with the number of cases.  Population buffers alternate by
 // step parity, so a chunk of an even number of steps can be captured once as a CUDA graph
@@ -55,7 +55,7 @@ __global__ void k_batch_pull_offsets(const lbm_lattice* __restrict__ lat, int K,
 }
 
 template <int VP, int G, bool OUT, bool AVG>
-__global__ void __launch_bounds__(128, VP == 8 ? 3 : 4) k_batch_plain(const BatchDesc B, int parity,
+__global__ void __launch_bounds__(128, VP == 8 ? 3 : 5) k_batch_plain(const BatchDesc B, int parity,
                                                                      const uint32_t* __restrict__ list, int nlist)
 {
     constexpr int PER_WARP = 32 / G;
@@ -69,40 +69,57 @@ __global__ void __launch_bounds__(128, VP == 8 ? 3 : 4) k_batch_plain(const Batc
     }
 }
 
-template <bool OUT, bool AVG>
-__global__ void __launch_bounds__(128, 3) k_batch_edge(const BatchDesc B, int parity, const uint32_t* __restrict__ list,
-                                                       int nlist)
+// One 32-cell pass of a batch's special entry e (64-cell segments): part 0 or 1 of it.
+template <bool OUT, bool UCOL, bool AVG, typename T>
+__device__ __forceinline__ void batch_cell_pass(const BatchDesc& B, int parity, uint32_t e, int part, int lane)
 {
-    constexpr int V = 2, SEG = 64;
-    const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), W = (int)((gridDim.x * blockDim.x) >> 5);
-    for (int w = gw; w < nlist; w += W) {
-        const BatchItem it = batch_item(B, parity, __ldg(list + w));
-        const lbm_lattice& L = B.lat[it.c];
-        const float scale = __ldg(B.scale + it.c);
-        int seg, y, z;
-        decode_row(it.id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
-        edge_segment<V, OUT, AVG, __half>(L, B.po[it.c], it.fs, it.fd, scale, 1.0f / scale, seg * SEG + lane * V, y, z,
-                                          lane);
-    }
+    constexpr int SEG = 64;
+    const BatchItem it = batch_item(B, parity, e);
+    const lbm_lattice& L = B.lat[it.c];
+    const float scale = __ldg(B.scale + it.c);
+    int seg, y, z;
+    decode_row(it.id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
+    const int xa = seg * SEG + part * 32;
+    if (xa >= L.pitch) return;                             // warp-uniform
+    cell_pass<SEG, OUT, UCOL, AVG, T>(L, reinterpret_cast<const T*>(it.fs), reinterpret_cast<T*>(it.fd), scale,
+                                      1.0f / scale, xa, y, z, lane, pass_flags(L, xa + lane, y, z));
+}
+
+// A warp pass over edge entries b and b+1 of a batch, 16 lanes each.  The two may be of cases whose
+// outlet cells sit at different places in their lanes, which edge_lane decides per group.
+template <bool OUT, bool AVG, typename T>
+__device__ __forceinline__ void batch_edge_pass(const BatchDesc& B, int parity, const uint32_t* __restrict__ list,
+                                                long long b, int nlist, int lane)
+{
+    constexpr int SEG = 64, G = 16;
+    const bool valid = b + lane / G < nlist;
+    const BatchItem it = batch_item(B, parity, __ldg(list + (valid ? b + lane / G : b)));
+    const lbm_lattice& L = B.lat[it.c];
+    const float scale = __ldg(B.scale + it.c);
+    int seg, y, z;
+    decode_row(it.id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
+    edge_lane<G, OUT, AVG, T>(L, B.po[it.c], reinterpret_cast<const T*>(it.fs), reinterpret_cast<T*>(it.fd), scale,
+                              1.0f / scale, seg * SEG + lane % G * 4, y, z, lane % G, valid);
 }
 
 template <bool OUT, bool UCOL, bool AVG>
-__global__ void __launch_bounds__(128, 4) k_batch_general(const BatchDesc B, int parity,
-                                                          const uint32_t* __restrict__ list, int nlist)
+__global__ void __launch_bounds__(128, 4) k_batch_cells(const BatchDesc B, int parity,
+                                                                 const uint32_t* __restrict__ special, int n_special)
 {
-    constexpr int V = 2, SEG = 64;
     const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), W = (int)((gridDim.x * blockDim.x) >> 5);
-    for (int w = gw; w < nlist; w += W) {
-        const BatchItem it = batch_item(B, parity, __ldg(list + w));
-        const lbm_lattice& L = B.lat[it.c];
-        const float scale = __ldg(B.scale + it.c);
-        int seg, y, z;
-        decode_row(it.id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
-        general_segment<V, OUT, UCOL, AVG, __half>(L, B.po[it.c], it.fs, it.fd, scale, 1.0f / scale,
-                                                   seg * SEG + lane * V, y, z, lane);
-    }
+    const long long W = ((long long)gridDim.x * blockDim.x) >> 5, total = 2LL * n_special;
+    for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += W)
+        batch_cell_pass<OUT, UCOL, AVG, __half>(B, parity, __ldg(special + (t >> 1)), (int)(t & 1), lane);
+}
+
+template <bool OUT, bool AVG>
+__global__ void __launch_bounds__(128, 4) k_batch_edge(const BatchDesc B, int parity,
+                                                                const uint32_t* __restrict__ edge, int n_edge)
+{
+    const int lane = threadIdx.x & 31;
+    const long long W = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long b = 2 * (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < n_edge; b += 2 * W)
+        batch_edge_pass<OUT, AVG, __half>(B, parity, edge, b, n_edge, lane);
 }
 
 template <bool AVG>
@@ -135,9 +152,9 @@ __global__ void k_batch_bc_rows(const BatchDesc B, int parity)
 // Persistent chunk: `nsteps` steps of the whole batch in ONE cooperative launch.  Every CTA stays
 // resident for the chunk; a step is two phases separated by grid barriers:
 //   phase 1  the step's segment tasks, statically interleaved over all warps of the grid in one
-//            task space [special | edge | plain groups]: a special or edge task is one 64-cell
-//            segment (the general / edge path, 2 cells per lane), a plain task four segments
-//            (8 lanes of 8 cells each); so every warp works through some of each kind and the
+//            task space [special | edge | plain groups]: a special task is half a 64-cell segment
+//            (one cell per lane), an edge task two segments (16 lanes of 4 cells each), a plain
+//            task four (8 lanes of 8 cells each); so every warp works through some of each kind and the
 //            latency-bound special segments run beside the bandwidth-bound plain ones;
 //   phase 2  the outlet rows of cases whose x = nx-2 and nx-1 lie in different segments, and on
 //            the chunk's last (output) step the solid segments' fields and the column means.
@@ -196,34 +213,20 @@ __device__ __forceinline__ void batch_tasks(const BatchDesc& B, int parity, cons
                                             int n_special, const uint32_t* __restrict__ edge, int n_edge,
                                             const uint32_t* __restrict__ plain, int n_plain)
 {
-    constexpr int V = 2, SEG = 64, VP = 8, G = 8, PER_WARP = 32 / G;
+    constexpr int VP = 8, G = 8, PER_WARP = 32 / G;
     const int lane = threadIdx.x & 31;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long W = ((long long)gridDim.x * blockDim.x) >> 5;
     const long long n_pgroups = (n_plain + PER_WARP - 1) / PER_WARP;
-    const long long total = (long long)n_special + n_edge + n_pgroups;
+    const long long ns = 2LL * n_special, ne = (n_edge + 1LL) / 2, total = ns + ne + n_pgroups;
     for (long long t = gw; t < total; t += W) {
         // populations are read with coherent loads (hcoh): this launch wrote them in earlier steps
-        if (t < n_special) {
-            const BatchItem it = batch_item(B, parity, __ldg(special + t));
-            const lbm_lattice& L = B.lat[it.c];
-            const float scale = __ldg(B.scale + it.c);
-            int seg, y, z;
-            decode_row(it.id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
-            general_segment<V, OUT, UCOL, AVG, hcoh>(L, B.po[it.c], reinterpret_cast<const hcoh*>(it.fs),
-                                                     reinterpret_cast<hcoh*>(it.fd), scale, 1.0f / scale,
-                                                     seg * SEG + lane * V, y, z, lane);
-        } else if (t < (long long)n_special + n_edge) {
-            const BatchItem it = batch_item(B, parity, __ldg(edge + (t - n_special)));
-            const lbm_lattice& L = B.lat[it.c];
-            const float scale = __ldg(B.scale + it.c);
-            int seg, y, z;
-            decode_row(it.id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
-            edge_segment<V, OUT, AVG, hcoh>(L, B.po[it.c], reinterpret_cast<const hcoh*>(it.fs),
-                                            reinterpret_cast<hcoh*>(it.fd), scale, 1.0f / scale, seg * SEG + lane * V,
-                                            y, z, lane);
+        if (t < ns) {
+            batch_cell_pass<OUT, UCOL, AVG, hcoh>(B, parity, __ldg(special + (t >> 1)), (int)(t & 1), lane);
+        } else if (t < ns + ne) {
+            batch_edge_pass<OUT, AVG, hcoh>(B, parity, edge, 2 * (t - ns), n_edge, lane);
         } else {
-            const long long b = (t - n_special - n_edge) * PER_WARP;
+            const long long b = (t - ns - ne) * PER_WARP;
             const int gl = lane % G, grp = lane / G;
             const bool valid = b + grp < n_plain;
             const BatchItem it = batch_item(B, parity, __ldg(plain + (valid ? b + grp : b)));

@@ -45,7 +45,8 @@ __device__ __forceinline__ void vstore(float* p, const float (&v)[V])
 template <int V>
 __device__ __forceinline__ void vstore_plain(float* p, const float (&v)[V])
 {
-    if constexpr (V == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    if constexpr (V == 1) *p = v[0];
+    else if constexpr (V == 2) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
     else if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
     else {
         reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
@@ -55,7 +56,8 @@ __device__ __forceinline__ void vstore_plain(float* p, const float (&v)[V])
 template <int V>
 __device__ __forceinline__ void vload_plain(float (&o)[V], const float* p)
 {
-    if constexpr (V == 2) { const float2 t = *reinterpret_cast<const float2*>(p); o[0] = t.x; o[1] = t.y; }
+    if constexpr (V == 1) o[0] = *p;
+    else if constexpr (V == 2) { const float2 t = *reinterpret_cast<const float2*>(p); o[0] = t.x; o[1] = t.y; }
     else {
 #pragma unroll
         for (int q = 0; q < V / 4; ++q) {
@@ -96,19 +98,6 @@ __device__ __forceinline__ uint32_t float2_to_half2_bits(float lo, float hi)
     return b;
 }
 
-template <int V>
-__device__ __forceinline__ void ldv(float (&o)[V], const __half* p)
-{
-    static_assert(V == 2 || V == 4, "16-bit general path moves 2 or 4 cells per lane");
-    if constexpr (V == 2) {
-        const float2 a = half2_bits_to_float2(__ldg(reinterpret_cast<const unsigned int*>(p)));
-        o[0] = a.x; o[1] = a.y;
-    } else {
-        const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
-        const float2 a = half2_bits_to_float2(t.x), b = half2_bits_to_float2(t.y);
-        o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-    }
-}
 __device__ __forceinline__ float ld1(const __half* p) { return __half2float(__ldg(p)); }
 
 // 16-bit storage read through coherent loads (ld.global.cg, served by L2): for a kernel that
@@ -118,56 +107,17 @@ __device__ __forceinline__ float ld1(const __half* p) { return __half2float(__ld
 struct __align__(2) hcoh {
     __half h;
 };
-template <int V>
-__device__ __forceinline__ void ldv(float (&o)[V], const hcoh* p)
-{
-    static_assert(V == 2 || V == 4, "16-bit general path moves 2 or 4 cells per lane");
-    if constexpr (V == 2) {
-        const float2 a = half2_bits_to_float2(__ldcg(reinterpret_cast<const unsigned int*>(p)));
-        o[0] = a.x; o[1] = a.y;
-    } else {
-        const uint2 t = __ldcg(reinterpret_cast<const uint2*>(p));
-        const float2 a = half2_bits_to_float2(t.x), b = half2_bits_to_float2(t.y);
-        o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-    }
-}
 __device__ __forceinline__ float ld1(const hcoh* p) { return __half2float(__ldcg(reinterpret_cast<const __half*>(p))); }
 
 // f (after the pull) from raw element values: identity for float storage.
-template <typename T, int V>
-__device__ __forceinline__ void raw_to_pop(float (&f)[V][Q], float inv_scale)
+template <typename T>
+__device__ __forceinline__ void raw_to_pop(float (&f)[Q], float inv_scale)
 {
     if constexpr (!std::is_same<T, float>::value) {
 #pragma unroll
-        for (int k = 0; k < V; ++k)
-#pragma unroll
-            for (int i = 0; i < Q; ++i) f[k][i] = fmaf(f[k][i], inv_scale, wgt(i));
+        for (int i = 0; i < Q; ++i) f[i] = fmaf(f[i], inv_scale, wgt(i));
     }
 }
-
-// Streaming store of direction I of V cells.
-template <int I, int V>
-__device__ __forceinline__ void stv(float* p, const float (&v)[V], float) { vstore<V>(p, v); }
-template <int I, int V>
-__device__ __forceinline__ void stv(__half* p, const float (&v)[V], float scale);
-template <int I, int V>
-__device__ __forceinline__ void stv(hcoh* p, const float (&v)[V], float scale)
-{
-    stv<I, V>(reinterpret_cast<__half*>(p), v, scale);
-}
-template <int I, int V>
-__device__ __forceinline__ void stv(__half* p, const float (&v)[V], float scale)
-{
-    static_assert(V == 2 || V == 4, "16-bit general path moves 2 or 4 cells per lane");
-    constexpr float w = wgt(I);
-    if constexpr (V == 2) {
-        __stcs(reinterpret_cast<unsigned int*>(p), float2_to_half2_bits((v[0] - w) * scale, (v[1] - w) * scale));
-    } else {
-        __stcs(reinterpret_cast<uint2*>(p), make_uint2(float2_to_half2_bits((v[0] - w) * scale, (v[1] - w) * scale),
-                                                       float2_to_half2_bits((v[2] - w) * scale, (v[3] - w) * scale)));
-    }
-}
-
 
 // Per-direction element offsets from a cell to its pull source in an interior row
 // (no wall, bed or lid involved): i*cells - cz(i)*ny*pitch - cy(i)*pitch; and in an open
@@ -184,6 +134,50 @@ __device__ __forceinline__ long long pull_offset(const PullOffsets& po, bool lid
 {
     if constexpr (cz(I) == -1) return lid ? po.lid[I] : po.d[I];
     else return po.d[I];
+}
+
+// Read-only loads that keep their order: the plain kernels issue all of a segment's loads before
+// the first shuffle or conversion waits for one.  The predicated ones leave `v` as it is in the
+// lanes where `on` is false.
+__device__ __forceinline__ void ld_ordered(uint32_t (&v)[1], const void* p)
+{
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v[0]) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered(uint32_t (&v)[2], const void* p)
+{
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered(uint32_t (&v)[4], const void* p)
+{
+    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered_if(bool on, uint32_t& v, const void* p)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+                 : "+r"(v) : "l"(p), "r"((uint32_t)on));
+}
+__device__ __forceinline__ void ld_ordered(uint16_t& v, const void* p)
+{
+    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered(float& v, const void* p)
+{
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered(float (&v)[2], const void* p)
+{
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered(float (&v)[4], const void* p)
+{
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void ld_ordered_if(bool on, float& v, const void* p)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"
+                 : "+f"(v) : "l"(p), "r"((uint32_t)on));
 }
 
 // One population of direction i (scalar; i need not be a compile-time constant).

@@ -8,90 +8,23 @@
 // Work lists are built over row segments of 32*cpl cells (cpl = cells_per_lane 2, 4 or 8:
 // 64, 128 or 256 cells), and pitch is a multiple of 8 so every 8-cell group is one aligned
 // 16-byte vector.
-//   k_rows_h_plain    plain segments: a lane moves VP = 8 (or 4) cells with one 16-byte (8-byte)
+//   k_rows_h_plain    plain segments: a lane moves VP = 4 (or 8) cells with one 8-byte (16-byte)
 //                     load/store per direction, 32*cpl/VP lanes per segment; the +-1 x
 //                     neighbours are one shuffle and VP/2 byte permutes on the packed halves;
 //                     the collision works on deviations directly (moments of f - w), two
-//                     cells at a time.
-//   k_rows_edge       edge segments and
-//   k_rows_h_general  special segments: the edge and general paths of fused_split.cuh with
-//                     T = __half, 2 cells per lane (4-byte accesses) for 64-cell segments,
-//                     else 4 (8-byte accesses) in one or two passes.
+//                     cells at a time in packed float32 (collide2).
+//   k_edge            edge segments (fused_edge.cuh) and
+//   k_cells           special segments (fused_cells.cuh), on populations.
 #pragma once
-
-// Regularized-BGK + Smagorinsky collision without body force, on deviations: `d` holds
-// raw storage values (f_i - w_i) * scale on entry and on exit.  Same update as collide():
-// with dr = rho - 1 and S = sum c c (f - w) (so that sum c c f = I/3 + S), the
-// non-equilibrium stress is Pi = S - rho u u - dr I/3, and the post-collision deviation is
-// w_i [ (A0 - 1) + c.B + c.C.c ].
-__device__ __forceinline__ void collide_dev(float (&d)[Q], float scale, float inv_scale, float tau0, float csmag2,
-                                            float& r, float& ux, float& uy, float& uz)
-{
-    const float s1 = d[1] + d[2], d1 = d[1] - d[2];
-    const float s3 = d[3] + d[4], d3 = d[3] - d[4];
-    const float s5 = d[5] + d[6], d5 = d[5] - d[6];
-    const float s7 = d[7] + d[8], d7 = d[7] - d[8];
-    const float s9 = d[9] + d[10], d9 = d[9] - d[10];
-    const float s11 = d[11] + d[12], d11 = d[11] - d[12];
-    const float s13 = d[13] + d[14], d13 = d[13] - d[14];
-    const float s15 = d[15] + d[16], d15 = d[15] - d[16];
-    const float s17 = d[17] + d[18], d17 = d[17] - d[18];
-    const float dr = (d[0] + (s1 + s3 + s5) + (s7 + s9 + s11) + (s13 + s15 + s17)) * inv_scale;
-    r = 1.0f + dr;
-    const float jx = (d1 + d7 + d9 + d11 + d13) * inv_scale;
-    const float jy = (d3 + d7 - d9 + d15 + d17) * inv_scale;
-    const float jz = (d5 + d11 - d13 + d15 - d17) * inv_scale;
-    const float sxx = (s1 + s7 + s9 + s11 + s13) * inv_scale;
-    const float syy = (s3 + s7 + s9 + s15 + s17) * inv_scale;
-    const float szz = (s5 + s11 + s13 + s15 + s17) * inv_scale;
-    const float sxy = (s7 - s9) * inv_scale, sxz = (s11 - s13) * inv_scale, syz = (s15 - s17) * inv_scale;
-
-    const float ir = 1.0f / r;
-    ux = jx * ir;
-    uy = jy * ir;
-    uz = jz * ir;
-    const float dr3 = dr * (1.0f / 3.0f);
-    const float pxx = sxx - r * ux * ux - dr3, pyy = syy - r * uy * uy - dr3, pzz = szz - r * uz * uz - dr3;
-    const float pxy = sxy - r * ux * uy, pxz = sxz - r * ux * uz, pyz = syz - r * uy * uz;
-
-    const float qn = sqrtf(pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * (pxy * pxy + pxz * pxz + pyz * pyz));
-    // tau0^2 and 18 sqrt(2) Cs^2 are rounded explicitly: they are lattice constants, and a compiler
-    // that hoists them out of a loop (or not) must not change how they fuse into what follows
-    const float tau0sq = mul_rn(tau0, tau0), smag = mul_rn(18.0f * 1.41421356f, csmag2);
-    const float tau = 0.5f * (tau0 + sqrtf(tau0sq + smag * qn * ir));
-    const float om = 1.0f / tau;
-    const float k1 = 1.0f - om;
-
-    const float usq = ux * ux + uy * uy + uz * uz;
-    const float A0 = dr - 1.5f * (r * usq + k1 * (pxx + pyy + pzz));
-    const float Bx = 3.0f * r * ux, By = 3.0f * r * uy, Bz = 3.0f * r * uz;
-    const float Cxx = 4.5f * (r * ux * ux + k1 * pxx);
-    const float Cyy = 4.5f * (r * uy * uy + k1 * pyy);
-    const float Czz = 4.5f * (r * uz * uz + k1 * pzz);
-    const float Cxy2 = 9.0f * (r * ux * uy + k1 * pxy);
-    const float Cxz2 = 9.0f * (r * ux * uz + k1 * pxz);
-    const float Cyz2 = 9.0f * (r * uy * uz + k1 * pyz);
-
-    const float w0 = wgt(0) * scale, w1 = wgt(1) * scale, w2 = wgt(7) * scale;
-    d[0] = w0 * A0;
-    float b;
-    b = A0 + Cxx;                 d[1] = w1 * (b + Bx);  d[2] = w1 * (b - Bx);
-    b = A0 + Cyy;                 d[3] = w1 * (b + By);  d[4] = w1 * (b - By);
-    b = A0 + Czz;                 d[5] = w1 * (b + Bz);  d[6] = w1 * (b - Bz);
-    b = A0 + Cxx + Cyy + Cxy2;    d[7] = w2 * (b + (Bx + By));  d[8] = w2 * (b - (Bx + By));
-    b = A0 + Cxx + Cyy - Cxy2;    d[9] = w2 * (b + (Bx - By));  d[10] = w2 * (b - (Bx - By));
-    b = A0 + Cxx + Czz + Cxz2;    d[11] = w2 * (b + (Bx + Bz)); d[12] = w2 * (b - (Bx + Bz));
-    b = A0 + Cxx + Czz - Cxz2;    d[13] = w2 * (b + (Bx - Bz)); d[14] = w2 * (b - (Bx - Bz));
-    b = A0 + Cyy + Czz + Cyz2;    d[15] = w2 * (b + (By + Bz)); d[16] = w2 * (b - (By + Bz));
-    b = A0 + Cyy + Czz - Cyz2;    d[17] = w2 * (b + (By - Bz)); d[18] = w2 * (b - (By - Bz));
-}
 
 // Pull of direction I for the VP cells (VP = 4 or 8) of a lane in an interior row, packed:
 // word j of h[I] holds cells 2j (low half) and 2j+1 (high half).  A +x mover takes element
 // x-1: word j = (high half of source word j-1, low half of source word j); word -1 is the
 // left lane's last word (at a segment's first lane: the 4-byte word just left of the
 // segment).  A -x mover takes element x+1 symmetrically, word VP/2 from the right lane.
-// G lanes share a segment (shuffles of width G).
+// G lanes share a segment (shuffles of width G).  All loads are issued, in order, before the
+// first shuffle waits for one: left to the compiler, the 16-bit kernel waited for early loads
+// with later ones not yet issued (VP = 8: 366 us against 404 on the 36M-cell reach).
 template <int VP> struct HVec;
 template <> struct HVec<4> {
     static __device__ __forceinline__ void load(uint32_t (&t)[2], const __half* p)
@@ -106,7 +39,7 @@ template <> struct HVec<4> {
 };
 // Stores are plain write-back stores: for this kernel they measured 2.7 % faster than
 // streaming (.cs) stores on reach36m, while the float32 kernels keep .cs stores (6 % slower
-// without); .cs, .nc.L1::no_allocate loads were 9-11 % slower than the default __ldg.
+// without); .cs, .nc.L1::no_allocate loads were 9-11 % slower than the default read-only ones.
 template <> struct HVec<8> {
     static __device__ __forceinline__ void load(uint32_t (&t)[4], const __half* p)
     {
@@ -136,29 +69,38 @@ __device__ __forceinline__ void hload(uint32_t (&t)[VP / 2], const hcoh* p)
 __device__ __forceinline__ uint32_t hword(const __half* p) { return __ldg(reinterpret_cast<const unsigned int*>(p)); }
 __device__ __forceinline__ uint32_t hword(const hcoh* p) { return __ldcg(reinterpret_cast<const unsigned int*>(p)); }
 
-template <int I, int VP, int G, typename T>
-__device__ __forceinline__ void hpull_dir(uint32_t (&h)[Q][VP / 2], const T* __restrict__ own_ptr,
-                                          const PullOffsets& po, int gl, bool lid)
+template <int I, int VP, typename T>
+__device__ __forceinline__ void hpull_load(uint32_t (&h)[Q][VP / 2], uint32_t (&e)[Q], const T* __restrict__ own_ptr,
+                                           const PullOffsets& po, int gl, int G, bool lid)
 {
-    constexpr int CXI = cx(I), NW = VP / 2;
     const T* src = own_ptr + pull_offset<I>(po, lid);
-    uint32_t t[NW];
-    hload<VP>(t, src);
-    if constexpr (CXI == 0) {
-#pragma unroll
-        for (int j = 0; j < NW; ++j) h[I][j] = t[j];
-    } else if constexpr (CXI == 1) {
-        uint32_t prev = __shfl_up_sync(0xffffffffu, t[NW - 1], 1, G);
-        if (gl == 0) prev = hword(src - 2);
-        h[I][0] = __byte_perm(prev, t[0], 0x5432);
-#pragma unroll
-        for (int j = 1; j < NW; ++j) h[I][j] = __byte_perm(t[j - 1], t[j], 0x5432);
+    e[I] = 0;
+    if constexpr (std::is_same<T, __half>::value) {
+        ld_ordered(h[I], src);
+        if constexpr (cx(I) == 1) ld_ordered_if(gl == 0, e[I], src - 2);
+        if constexpr (cx(I) == -1) ld_ordered_if(gl == G - 1, e[I], src + VP);
     } else {
-        uint32_t next = __shfl_down_sync(0xffffffffu, t[0], 1, G);
-        if (gl == G - 1) next = hword(src + VP);
+        hload<VP>(h[I], src);
+        if constexpr (cx(I) == 1) if (gl == 0) e[I] = hword(src - 2);
+        if constexpr (cx(I) == -1) if (gl == G - 1) e[I] = hword(src + VP);
+    }
+}
+template <int I, int VP, int G>
+__device__ __forceinline__ void hpull_shift(uint32_t (&h)[Q][VP / 2], const uint32_t (&e)[Q], int gl)
+{
+    constexpr int NW = VP / 2;
+    if constexpr (cx(I) == 1) {
+        uint32_t prev = __shfl_up_sync(0xffffffffu, h[I][NW - 1], 1, G);
+        if (gl == 0) prev = e[I];
 #pragma unroll
-        for (int j = 0; j < NW - 1; ++j) h[I][j] = __byte_perm(t[j], t[j + 1], 0x5432);
-        h[I][NW - 1] = __byte_perm(t[NW - 1], next, 0x5432);
+        for (int j = NW - 1; j > 0; --j) h[I][j] = __byte_perm(h[I][j - 1], h[I][j], 0x5432);
+        h[I][0] = __byte_perm(prev, h[I][0], 0x5432);
+    } else if constexpr (cx(I) == -1) {
+        uint32_t next = __shfl_down_sync(0xffffffffu, h[I][0], 1, G);
+        if (gl == G - 1) next = e[I];
+#pragma unroll
+        for (int j = 0; j < NW - 1; ++j) h[I][j] = __byte_perm(h[I][j], h[I][j + 1], 0x5432);
+        h[I][NW - 1] = __byte_perm(h[I][NW - 1], next, 0x5432);
     }
 }
 template <int VP, int G, typename T, int... Is>
@@ -166,7 +108,9 @@ __device__ __forceinline__ void hpull_all(std::integer_sequence<int, Is...>, uin
                                           const T* __restrict__ own_ptr, const PullOffsets& po, int gl,
                                           bool lid)
 {
-    (hpull_dir<Is, VP, G, T>(h, own_ptr, po, gl, lid), ...);
+    uint32_t e[Q];
+    (hpull_load<Is, VP, T>(h, e, own_ptr, po, gl, G, lid), ...);
+    (hpull_shift<Is, VP, G>(h, e, gl), ...);
 }
 
 // One plain segment (row-segment id `id`) for the G lanes of a group: lane gl of the group
@@ -189,16 +133,14 @@ __device__ __forceinline__ void h_plain_segment(const lbm_lattice& L, const Pull
     float R[VP], UX[VP], UY[VP], UZ[VP];
 #pragma unroll
     for (int p = 0; p < NW; ++p) {
-        float a[Q], c[Q];
+        float2 d[Q], r2, ux2, uy2, uz2;
 #pragma unroll
-        for (int i = 0; i < Q; ++i) {
-            const float2 v = half2_bits_to_float2(h[i][p]);
-            a[i] = v.x; c[i] = v.y;
-        }
-        collide_dev(a, scale, inv_scale, L.tau0, L.csmag2, R[2 * p], UX[2 * p], UY[2 * p], UZ[2 * p]);
-        collide_dev(c, scale, inv_scale, L.tau0, L.csmag2, R[2 * p + 1], UX[2 * p + 1], UY[2 * p + 1], UZ[2 * p + 1]);
+        for (int i = 0; i < Q; ++i) d[i] = half2_bits_to_float2(h[i][p]);
+        collide2<true, AVG>(d, scale, inv_scale, L.tau0, L.csmag2, r2, ux2, uy2, uz2);
+        R[2 * p] = r2.x; UX[2 * p] = ux2.x; UY[2 * p] = uy2.x; UZ[2 * p] = uz2.x;
+        R[2 * p + 1] = r2.y; UX[2 * p + 1] = ux2.y; UY[2 * p + 1] = uy2.y; UZ[2 * p + 1] = uz2.y;
 #pragma unroll
-        for (int i = 0; i < Q; ++i) h[i][p] = float2_to_half2_bits(a[i], c[i]);
+        for (int i = 0; i < Q; ++i) h[i][p] = float2_to_half2_bits(d[i].x, d[i].y);
     }
     if (!store) return;
 #pragma unroll
@@ -215,9 +157,13 @@ __device__ __forceinline__ void h_plain_segment(const lbm_lattice& L, const Pull
 // Plain list over segments of VP*G cells: a warp takes 32/G consecutive list entries per
 // pass, G lanes (VP cells each) per segment.  In the last pass, groups past the end of the
 // list repeat the pass's first segment and store nothing (every lane still takes part in
-// the shuffles).
+// the shuffles).  One pass per warp unless the grid is held down (lbm_tile.ctas_per_sm): CTAs
+// that come and go sweep the list in order, 4 % faster than a resident grid striding over it
+// (347 against 360 us on the 27.3M plain cells of the 36M-cell reach, 5.98 TB/s of 76 B a cell).
+// VP = 4 keeps 20 warps per SM (96 registers), VP = 8 12 (168, 345 us there, but half the warps
+// where a case is small).
 template <int VP, int G, bool OUT, bool AVG>
-__global__ void __launch_bounds__(128, VP == 8 ? 3 : 4) k_rows_h_plain(const lbm_lattice L, const PullOffsets po,
+__global__ void __launch_bounds__(128, VP == 8 ? 3 : 5) k_rows_h_plain(const lbm_lattice L, const PullOffsets po,
                                                                       const uint32_t* __restrict__ list, int nlist,
                                                                       const __half* __restrict__ fs,
                                                                       __half* __restrict__ fd, float scale)

@@ -129,37 +129,42 @@ __device__ __forceinline__ void pull_fixups(std::integer_sequence<int, Is...>, f
 // fetch the one halo element.  At the x
 // edges and in padding lanes the values are fixed up (or discarded) afterwards; every
 // address stays inside the population array because an interior row has rows on both sides.
-template <int I, int V, typename T>
-__device__ __forceinline__ void pull_fast_dir(float (&f)[V][Q], const T* __restrict__ own_ptr,
-                                              const PullOffsets& po, int lane, bool lid)
+template <int I, int V>
+__device__ __forceinline__ void pull_fast_load(float (&t)[Q][V], float (&e)[Q], const float* __restrict__ own_ptr,
+                                               const PullOffsets& po, int lane, bool lid)
 {
-    constexpr int CXI = cx(I);
-    const T* src = own_ptr + pull_offset<I>(po, lid);
-    float t[V];
-    ldv<V>(t, src);
-    if constexpr (CXI == 0) {
+    const float* src = own_ptr + pull_offset<I>(po, lid);
+    e[I] = 0.f;
+    ld_ordered(t[I], src);
+    if constexpr (cx(I) == 1) ld_ordered_if(lane == 0, e[I], src - 1);
+    if constexpr (cx(I) == -1) ld_ordered_if(lane == 31, e[I], src + V);
+}
+template <int I, int V>
+__device__ __forceinline__ void pull_fast_shift(float (&f)[V][Q], const float (&t)[Q][V], const float (&e)[Q], int lane)
+{
+    if constexpr (cx(I) == 0) {
 #pragma unroll
-        for (int k = 0; k < V; ++k) f[k][I] = t[k];
-    } else if constexpr (CXI == 1) {
-        float h = __shfl_up_sync(0xffffffffu, t[V - 1], 1);
-        if (lane == 0) h = ld1(src - 1);
-        f[0][I] = h;
+        for (int k = 0; k < V; ++k) f[k][I] = t[I][k];
+    } else if constexpr (cx(I) == 1) {
+        const float h = __shfl_up_sync(0xffffffffu, t[I][V - 1], 1);
+        f[0][I] = lane == 0 ? e[I] : h;
 #pragma unroll
-        for (int k = 1; k < V; ++k) f[k][I] = t[k - 1];
+        for (int k = 1; k < V; ++k) f[k][I] = t[I][k - 1];
     } else {
-        float h = __shfl_down_sync(0xffffffffu, t[0], 1);
-        if (lane == 31) h = ld1(src + V);
+        const float h = __shfl_down_sync(0xffffffffu, t[I][0], 1);
 #pragma unroll
-        for (int k = 0; k < V - 1; ++k) f[k][I] = t[k + 1];
-        f[V - 1][I] = h;
+        for (int k = 0; k < V - 1; ++k) f[k][I] = t[I][k + 1];
+        f[V - 1][I] = lane == 31 ? e[I] : h;
     }
 }
-template <int V, typename T, int... Is>
+template <int V, int... Is>
 __device__ __forceinline__ void pull_fast_all(std::integer_sequence<int, Is...>, float (&f)[V][Q],
-                                              const T* __restrict__ own_ptr, const PullOffsets& po, int lane,
+                                              const float* __restrict__ own_ptr, const PullOffsets& po, int lane,
                                               bool lid = false)
 {
-    (pull_fast_dir<Is, V, T>(f, own_ptr, po, lane, lid), ...);
+    float t[Q][V], e[Q];
+    (pull_fast_load<Is, V>(t, e, own_ptr, po, lane, lid), ...);
+    (pull_fast_shift<Is, V>(f, t, e, lane), ...);
 }
 
 template <int V, bool OUT, bool UCOL, bool AVG>
@@ -240,7 +245,7 @@ __global__ void __launch_bounds__(128, V == 4 ? 3 : 4) k_fused(const lbm_lattice
             if (!__any_sync(0xffffffffu, flany & (FLAG_SOLID | FLAG_WALLFN | FLAG_FORCE))) {
 #pragma unroll
                 for (int k = 0; k < V; ++k)
-                    collide(f[k], 0.f, 0.f, 0.f, L.tau0, L.csmag2, R[k], UX[k], UY[k], UZ[k]);
+                    collide<false>(f[k], 0.f, 0.f, 0.f, L.tau0, L.csmag2, R[k], UX[k], UY[k], UZ[k]);
             } else {
 #pragma unroll
                 for (int k = 0; k < V; ++k) {
@@ -263,17 +268,17 @@ __global__ void __launch_bounds__(128, V == 4 ? 3 : 4) k_fused(const lbm_lattice
                             fy = L.Fy[c] * L.force_scale;
                             fz = L.Fz[c] * L.force_scale;
                         }
-                        collide(f[k], fx, fy, fz, L.tau0, L.csmag2, R[k], UX[k], UY[k], UZ[k]);
+                        collide<true>(f[k], fx, fy, fz, L.tau0, L.csmag2, R[k], UX[k], UY[k], UZ[k]);
                     }
                 }
             }
             // inlet (x=0 from x=1) and outlet (x=nx-1 from x=nx-2), both inside this lane
             if (x0 == 0 && !(fl[0] & FLAG_SOLID) && !(fl[1] & FLAG_SOLID))
-                nebb<true>(f[1], f[0], L.uin[y + (long long)L.ny * z], L.rho_out);
+                nebb(true, f[1], f[0], L.uin[y + (long long)L.ny * z], L.rho_out);
 #pragma unroll
             for (int k = 1; k < V; ++k)
                 if (x0 + k == L.nx - 1 && !(fl[k] & FLAG_SOLID) && !(fl[k - 1] & FLAG_SOLID))
-                    nebb<false>(f[k - 1], f[k], 0.f, L.rho_out);
+                    nebb(false, f[k - 1], f[k], 0.f, L.rho_out);
 
             if (active) {
 #pragma unroll

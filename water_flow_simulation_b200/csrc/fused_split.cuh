@@ -12,15 +12,13 @@
 //   solid   -- every cell solid (or padding);
 //   special -- everything else (walls, bed, lid, banks, hulls, forcing).
 // A step then runs
-//   k_rows<PLAIN>   over the plain list: 19 V-wide pulls at constant offsets (the +-1 x
+//   k_rows          over the plain list: 19 V-wide pulls at constant offsets (the +-1 x
 //                   neighbours by warp shuffle), collision with no force, 19 V-wide
 //                   streaming stores -- no flag word is read; this is where the cells are;
-//   k_rows_edge     over the edge list: the plain pull, the x-edge copies, the inlet and
-//                   outlet extrapolation and rest-state padding, still without flag words;
-//   k_rows<SPECIAL> over the special list: the general path of fused_reg.cuh (flag words,
-//                   y-wall/bed/lid rows, bounce-back, x edges, wall function, forcing,
-//                   inlet/outlet), compiled separately so its register needs do not
-//                   throttle the plain kernel;
+//   k_cells         (fused_cells.cuh) over the special list: flag words, y walls, bed, lid,
+//                   bounce-back, x edges, wall function, forcing, inlet/outlet, one cell per lane;
+//   k_edge          (fused_edge.cuh) over the edge list: the plain pull, the x-edge copies, the
+//                   inlet and outlet extrapolation and rest-state padding, without flag words;
 //   k_solid_out     on output steps only: the fields of solid segments;
 //   k_column_mean   on output steps with the column-mean wall model: the depth-mean speed
 //                   of every (y, x) column, summed over z in order.
@@ -112,25 +110,25 @@ __global__ void __launch_bounds__(1024) k_compact(const uint8_t* __restrict__ cl
     if (tid < NC) counts[tid] = base[tid];
 }
 
-// Streaming stores of the V cells' 19 populations (T = float or 16-bit storage).
-template <int I, int V, typename T>
-__device__ __forceinline__ void store_pop(T* p, const float (&f)[V][Q], float scale)
+// Streaming stores of the V cells' 19 populations.
+template <int I, int V>
+__device__ __forceinline__ void store_pop(float* p, const float (&f)[V][Q])
 {
     float v[V];
 #pragma unroll
     for (int k = 0; k < V; ++k) v[k] = f[k][I];
-    stv<I, V>(p, v, scale);
+    vstore<V>(p, v);
 }
-template <int V, typename T, int... Is>
-__device__ __forceinline__ void store_pops(std::integer_sequence<int, Is...>, T* fd, long long S, long long own,
-                                           const float (&f)[V][Q], float scale)
+template <int V, int... Is>
+__device__ __forceinline__ void store_pops(std::integer_sequence<int, Is...>, float* fd, long long S, long long own,
+                                           const float (&f)[V][Q])
 {
-    (store_pop<Is, V>(fd + (long long)Is * S + own, f, scale), ...);
+    (store_pop<Is, V>(fd + (long long)Is * S + own, f), ...);
 }
 
 // Output-step fields of V cells and, with AVG, their time-average sums
-// (floodsim/reach3d.py:443-451: ux, uy, uz, rho, speed, ux^2).
-template <int V, bool AVG>
+// (floodsim/reach3d.py:443-451: ux, uy, uz, rho, speed, ux^2).  UX2: as in collide().
+template <int V, bool AVG, bool UX2 = (V > 1)>
 __device__ __forceinline__ void store_fields(const lbm_lattice& L, long long own, const float (&R)[V],
                                              const float (&UX)[V], const float (&UY)[V], const float (&UZ)[V])
 {
@@ -152,28 +150,11 @@ __device__ __forceinline__ void store_fields(const lbm_lattice& L, long long own
         WFS_ACC(1, UY[k])
         WFS_ACC(2, UZ[k])
         WFS_ACC(3, R[k])
-        WFS_ACC(4, sqrtf(UX[k] * UX[k] + UY[k] * UY[k] + UZ[k] * UZ[k]))
+        WFS_ACC(4, sqrtf(fma_rn(UZ[k], UZ[k], UX2 ? fma_rn(UY[k], UY[k], mul_rn(UX[k], UX[k]))
+                                              : fma_rn(UX[k], UX[k], mul_rn(UY[k], UY[k])))))
         WFS_ACC(5, UX[k] * UX[k])
 #undef WFS_ACC
     }
-}
-
-// Outlet cell x = nx-1 as the first cell of a lane whose left neighbour lane holds x = nx-2:
-// that lane's post-collision populations arrive by shuffle, so the extrapolation uses the
-// same unrounded values as when both cells share a lane.  (When x = nx-2 is in the previous
-// segment -- nx-1 a multiple of the segment length -- a separate pass does it.)  Called by
-// all lanes of the warp.
-template <int V>
-__device__ __forceinline__ void outlet_from_left_lane(float (&f)[V][Q], const lbm_lattice& L, int x0, int lane,
-                                                      bool own_solid, bool last_solid)
-{
-    const bool here = x0 == L.nx - 1 && lane > 0;
-    if (!__any_sync(0xffffffffu, here)) return;
-    float g[Q];
-#pragma unroll
-    for (int i = 0; i < Q; ++i) g[i] = __shfl_up_sync(0xffffffffu, f[V - 1][i], 1);
-    const bool left_solid = __shfl_up_sync(0xffffffffu, last_solid, 1);
-    if (here && !own_solid && !left_solid) nebb<false>(g, f[0], 0.f, L.rho_out);
 }
 
 // Relaxation time at zero strain of column x: tau0, or inside the optional outlet sponge
@@ -186,219 +167,46 @@ __device__ __forceinline__ float sponge_tau0(const lbm_lattice& L, int x)
     return __fadd_rn(L.tau0, __fmul_rn(__fsub_rn(L.sponge_tau, L.tau0), __fmul_rn(s, s)));
 }
 
-// The general path for the V cells from x0 of row (y, z): flag words, y-wall/bed/lid rows,
-// bounce-back, x edges, wall function, forcing, inlet/outlet, then the stores.  T is the
-// population element type; `scale` / `inv_scale` are the 16-bit storage scale and its inverse.
-template <int V, bool OUT, bool UCOL, bool AVG, typename T>
-__device__ __forceinline__ void general_segment(const lbm_lattice& L, const PullOffsets& po, const T* __restrict__ fs,
-                                                T* __restrict__ fd, float scale, float inv_scale, int x0, int y, int z,
-                                                int lane)
-{
-    const long long S = L.cells;
-    const long long rowc = ((long long)z * L.ny + y) * L.pitch;
-    const long long own = rowc + x0;
-    float f[V][Q];
-    float R[V], UX[V], UY[V], UZ[V];
-    const bool active = x0 < L.pitch;
-    const int x0c = active ? x0 : L.pitch - V;
-    PullCtxT<T> pc{fs, S, rowc, rowc + x0c, x0, x0c, y, z, lane};
-    uint32_t fl[V];
-    Vec<V>::loadu(fl, L.flags + pc.own);
-    const bool interior = y >= 1 && y <= L.ny - 2 && z >= 1 && z <= L.nz - 2;
-    uint32_t rwm = 0;
-    if (interior) pull_fast_all<V>(std::make_integer_sequence<int, Q>{}, f, fs + pc.own, po, lane);
-    else rwm = pull_rows<V>(std::make_integer_sequence<int, Q>{}, f, L, pc);
-    uint32_t flany = 0;
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-        if (!active) fl[k] = FLAG_GHOST | FLAG_SOLID;
-        flany |= fl[k];
-    }
-    pull_fixups<V>(std::make_integer_sequence<int, Q>{}, f, L, pc, fl, flany & FLAG_WALLS & ~rwm);
-    raw_to_pop<T, V>(f, inv_scale);
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-        const uint32_t fk = fl[k];
-        const long long c = own + k;
-        if (fk & FLAG_SOLID) {
-#pragma unroll
-            for (int i = 0; i < Q; ++i) f[k][i] = wgt(i);
-            R[k] = 1.f; UX[k] = 0.f; UY[k] = 0.f; UZ[k] = 0.f;
-        } else {
-            if (fk & FLAG_WALLFN) {
-                float U;
-                if constexpr (UCOL) U = (fk & FLAG_BEDWALL) ? L.colU[(long long)y * L.pitch + x0 + k] : 0.f;
-                else U = L.uref[c];
-                wall_function(f[k], fk & FLAG_WALLS, L.cfw[c], L.ux[c], L.uy[c], L.uz[c], L.rho[c], U);
-            }
-            float fx = 0.f, fy = 0.f, fz = 0.f;
-            if (fk & FLAG_FORCE) {
-                fx = L.Fx[c] * L.force_scale;
-                fy = L.Fy[c] * L.force_scale;
-                fz = L.Fz[c] * L.force_scale;
-            }
-            collide(f[k], fx, fy, fz, sponge_tau0(L, x0 + k), L.csmag2, R[k], UX[k], UY[k], UZ[k]);
-        }
-    }
-    // inlet (x=0 from x=1) and outlet (x=nx-1 from x=nx-2), both inside this lane
-    if (x0 == 0 && !(fl[0] & FLAG_SOLID) && !(fl[1] & FLAG_SOLID))
-        nebb<true>(f[1], f[0], L.uin[y + (long long)L.ny * z], L.rho_out);
-#pragma unroll
-    for (int k = 1; k < V; ++k)
-        if (x0 + k == L.nx - 1 && !(fl[k] & FLAG_SOLID) && !(fl[k - 1] & FLAG_SOLID))
-            nebb<false>(f[k - 1], f[k], 0.f, L.rho_out);
-    outlet_from_left_lane<V>(f, L, x0, lane, (fl[0] & FLAG_SOLID) != 0, (fl[V - 1] & FLAG_SOLID) != 0);
-    if (!active) return;
-    if constexpr (!OUT) {                                 // the wall function reads these next step
-#pragma unroll
-        for (int k = 0; k < V; ++k)
-            if (fl[k] & FLAG_WALLFN) {
-                L.rho[own + k] = R[k]; L.ux[own + k] = UX[k]; L.uy[own + k] = UY[k]; L.uz[own + k] = UZ[k];
-            }
-    } else {
-        bool bad = false;
-#pragma unroll
-        for (int k = 0; k < V; ++k) bad |= !(fl[k] & FLAG_SOLID) && !(R[k] > 0.f && R[k] < 3.4e38f);
-        if (bad) atomicOr(L.status, 1);
-    }
-    store_pops<V>(std::make_integer_sequence<int, Q>{}, fd, S, own, f, scale);
-    if constexpr (OUT) store_fields<V, AVG>(L, own, R, UX, UY, UZ);
-}
-
-// Special list: each list segment of PASSES*32*V cells in PASSES warp passes through the
-// general path.
-// Occupancy: the 16-bit V = 2 variant fits 128 registers without spills, so 4 CTAs (16 warps)
-// per SM hide more of its dependent flag -> pull -> wall-function latency (9.6 % less time for
-// the special segments of reach36m than at 3 CTAs); the float32 one would spill there.
-template <int V, int PASSES, bool OUT, bool UCOL, bool AVG, typename T>
-__global__ void __launch_bounds__(128, V <= 2 ? (std::is_same<T, __half>::value ? 4 : 3) : 2)
-    k_general(const lbm_lattice L, const PullOffsets po,
-                                                    const uint32_t* __restrict__ list, int nlist,
-                                                    const T* __restrict__ fs, T* __restrict__ fd, float scale)
-{
-    constexpr int SEG = PASSES * 32 * V, PASS = 32 * V;
-    const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), W = (int)((gridDim.x * blockDim.x) >> 5);
-    const int nseg = (L.pitch + SEG - 1) / SEG;
-    const float inv_scale = 1.0f / scale;
-    uint32_t next = gw < nlist ? __ldg(list + gw) : 0u;          // list entries are fetched one ahead
-    for (int w = gw; w < nlist; w += W) {
-        const uint32_t id = next;
-        if (w + W < nlist) next = __ldg(list + w + W);
-        int seg, y, z;
-        decode_row(id, nseg, L.ny, seg, y, z);
-#pragma unroll 1
-        for (int part = 0; part < PASSES; ++part) {
-            const int xa = seg * SEG + part * PASS;
-            if (xa >= L.pitch) break;                                  // warp-uniform
-            general_segment<V, OUT, UCOL, AVG, T>(L, po, fs, fd, scale, inv_scale, xa + lane * V, y, z, lane);
-        }
-    }
-}
-
-// Edge segment (first or last of an open interior row, no flags set below nx): the plain pull,
-// then the x-edge copies (a direction whose source lies outside [0, nx) keeps the cell's own
-// population, floodsim/lbm3d.py:48-49), collision without force, the inlet at x = 0 and the
-// outlet at x = nx-1 (when x = nx-2 is in the same lane), and padding cells (x >= nx) held at
-// rest.  Loads stay inside the population array: an interior row has rows on both sides.
-template <int V, bool OUT, bool AVG, typename T>
-__device__ __forceinline__ void edge_segment(const lbm_lattice& L, const PullOffsets& po, const T* __restrict__ fs,
-                                             T* __restrict__ fd, float scale, float inv_scale, int x0, int y, int z,
-                                             int lane)
-{
-    const long long S = L.cells;
-    const long long rowc = ((long long)z * L.ny + y) * L.pitch;
-    const bool active = x0 < L.pitch;
-    const int x0c = active ? x0 : L.pitch - V;
-    const long long own = rowc + x0c;
-    float f[V][Q];
-    float R[V], UX[V], UY[V], UZ[V];
-    pull_fast_all<V>(std::make_integer_sequence<int, Q>{}, f, fs + own, po, lane, z == L.nz - 1);
-    PullCtxT<T> pc{fs, S, rowc, own, x0, x0c, y, z, lane};
-    const bool edge = (x0 == 0) || (x0 <= L.nx - 1 && L.nx - 1 < x0 + V);
-    if (edge) pull_edges<V>(std::make_integer_sequence<int, Q>{}, f, L, pc);
-    raw_to_pop<T, V>(f, inv_scale);
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-        if (x0 + k >= L.nx) {
-#pragma unroll
-            for (int i = 0; i < Q; ++i) f[k][i] = wgt(i);
-            R[k] = 1.f; UX[k] = 0.f; UY[k] = 0.f; UZ[k] = 0.f;
-        } else {
-            collide(f[k], 0.f, 0.f, 0.f, L.tau0, L.csmag2, R[k], UX[k], UY[k], UZ[k]);
-        }
-    }
-    if (x0 == 0) nebb<true>(f[1], f[0], L.uin[y + (long long)L.ny * z], L.rho_out);
-#pragma unroll
-    for (int k = 1; k < V; ++k)
-        if (x0 + k == L.nx - 1) nebb<false>(f[k - 1], f[k], 0.f, L.rho_out);
-    outlet_from_left_lane<V>(f, L, x0, lane, false, false);
-    if (!active) return;
-    store_pops<V>(std::make_integer_sequence<int, Q>{}, fd, S, own, f, scale);
-    if constexpr (OUT) {
-        store_fields<V, AVG>(L, own, R, UX, UY, UZ);
-        bool bad = false;
-#pragma unroll
-        for (int k = 0; k < V; ++k) bad |= !(R[k] > 0.f && R[k] < 3.4e38f);
-        if (bad) atomicOr(L.status, 1);
-    }
-}
-
-// Edge list: each list segment of PASSES*32*V cells in PASSES warp passes of 32*V cells.
-template <int V, int PASSES, bool OUT, bool AVG, typename T>
-__global__ void __launch_bounds__(128, 3) k_rows_edge(const lbm_lattice L, const PullOffsets po,
-                                                      const uint32_t* __restrict__ list, int nlist,
-                                                      const T* __restrict__ fs, T* __restrict__ fd, float scale)
-{
-    constexpr int SEG = PASSES * 32 * V;
-    const int lane = threadIdx.x & 31;
-    const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), W = (int)((gridDim.x * blockDim.x) >> 5);
-    const int nseg = (L.pitch + SEG - 1) / SEG;
-    const float inv_scale = 1.0f / scale;
-    for (int w = gw; w < nlist; w += W) {
-        int seg, y, z;
-        decode_row(__ldg(list + w), nseg, L.ny, seg, y, z);
-#pragma unroll 1
-        for (int part = 0; part < PASSES; ++part) {
-            const int xa = seg * SEG + part * 32 * V;
-            if (xa >= L.pitch) break;                                  // warp-uniform
-            edge_segment<V, OUT, AVG, T>(L, po, fs, fd, scale, inv_scale, xa + lane * V, y, z, lane);
-        }
-    }
-}
-
-template <int V, bool PLAIN, bool OUT, bool UCOL, bool AVG>
-__global__ void __launch_bounds__(128, PLAIN ? 3 : 2) k_rows(const lbm_lattice L, const PullOffsets po,
-                                                             const uint32_t* __restrict__ list, int nlist,
-                                                             const float* __restrict__ fs, float* __restrict__ fd)
+// Plain list: a warp pass per segment of 32*V cells, one pass per warp unless the grid is held
+// down (lbm_tile.ctas_per_sm).  Bound by HBM: with V = 4, 16 warps per SM (118 registers) and all
+// of a pass's 19 16-byte loads issued before anything waits, 155 KB are in flight per SM, and CTAs
+// that come and go sweep the list in order; 605 us on the 36M-cell reach, against 734 for a
+// resident grid of 12 warps per SM and the scalar collision.
+template <int V, bool OUT, bool AVG>
+__global__ void __launch_bounds__(128, V == 4 ? 4 : 6) k_rows(const lbm_lattice L, const PullOffsets po,
+                                                              const uint32_t* __restrict__ list, int nlist,
+                                                              const float* __restrict__ fs, float* __restrict__ fd)
 {
     constexpr int SEG = 32 * V;
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), W = (int)((gridDim.x * blockDim.x) >> 5);
     const int nseg = (L.pitch + SEG - 1) / SEG;
     const long long S = L.cells;
-    uint32_t next = gw < nlist ? __ldg(list + gw) : 0u;          // list entries are fetched one ahead
     for (int w = gw; w < nlist; w += W) {
-        const uint32_t id = next;
-        if (w + W < nlist) next = __ldg(list + w + W);
         int seg, y, z;
-        decode_row(id, nseg, L.ny, seg, y, z);
-        const int x0 = seg * SEG + lane * V;
-        {
-            const long long own = ((long long)z * L.ny + y) * L.pitch + x0;
-            float f[V][Q];
-            float R[V], UX[V], UY[V], UZ[V];
-            pull_fast_all<V>(std::make_integer_sequence<int, Q>{}, f, fs + own, po, lane, z == L.nz - 1);
+        decode_row(__ldg(list + w), nseg, L.ny, seg, y, z);
+        const long long own = ((long long)z * L.ny + y) * L.pitch + seg * SEG + lane * V;
+        float f[V][Q];
+        float R[V], UX[V], UY[V], UZ[V];
+        pull_fast_all<V>(std::make_integer_sequence<int, Q>{}, f, fs + own, po, lane, z == L.nz - 1);
 #pragma unroll
-            for (int k = 0; k < V; ++k) collide(f[k], 0.f, 0.f, 0.f, L.tau0, L.csmag2, R[k], UX[k], UY[k], UZ[k]);
-            store_pops<V>(std::make_integer_sequence<int, Q>{}, fd, S, own, f, 1.f);
-            if constexpr (OUT) {
-                store_fields<V, AVG>(L, own, R, UX, UY, UZ);
-                bool bad = false;
+        for (int k = 0; k < V; k += 2) {
+            float2 d[Q], r2, ux2, uy2, uz2;
 #pragma unroll
-                for (int k = 0; k < V; ++k) bad |= !(R[k] > 0.f && R[k] < 3.4e38f);
-                if (bad) atomicOr(L.status, 1);
-            }
+            for (int i = 0; i < Q; ++i) d[i] = make_float2(f[k][i], f[k + 1][i]);
+            collide2<false, AVG>(d, 1.f, 1.f, L.tau0, L.csmag2, r2, ux2, uy2, uz2);
+#pragma unroll
+            for (int i = 0; i < Q; ++i) { f[k][i] = d[i].x; f[k + 1][i] = d[i].y; }
+            R[k] = r2.x; UX[k] = ux2.x; UY[k] = uy2.x; UZ[k] = uz2.x;
+            R[k + 1] = r2.y; UX[k + 1] = ux2.y; UY[k + 1] = uy2.y; UZ[k + 1] = uz2.y;
+        }
+        store_pops<V>(std::make_integer_sequence<int, Q>{}, fd, S, own, f);
+        if constexpr (OUT) {
+            store_fields<V, AVG>(L, own, R, UX, UY, UZ);
+            bool bad = false;
+#pragma unroll
+            for (int k = 0; k < V; ++k) bad |= !(R[k] > 0.f && R[k] < 3.4e38f);
+            if (bad) atomicOr(L.status, 1);
         }
     }
 }

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(32 * (C + 1), C == 8 ? 2 : 1) k_fused_tma(cons
                 fy = L.Fy[c] * L.force_scale;
                 fz = L.Fz[c] * L.force_scale;
             }
-            collide(f, fx, fy, fz, L.tau0, L.csmag2, R, UX, UY, UZ);
+            collide<true>(f, fx, fy, fz, L.tau0, L.csmag2, R, UX, UY, UZ);
         }
 
         // inlet: x=0 (lane 0 of warp 0, segment 0) from x=1 (lane 1)
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(32 * (C + 1), C == 8 ? 2 : 1) k_fused_tma(cons
             for (int i = 0; i < Q; ++i) g[i] = __shfl_down_sync(0xffffffffu, f[i], 1);
             const uint32_t f1 = __shfl_down_sync(0xffffffffu, fk, 1);
             if (lane == 0 && !(fk & FLAG_SOLID) && !(f1 & FLAG_SOLID))
-                nebb<true>(g, f, L.uin[id.y + (long long)L.ny * id.z], L.rho_out);
+                nebb(true, g, f, L.uin[id.y + (long long)L.ny * id.z], L.rho_out);
         }
         // outlet: x=nx-1 from x=nx-2 (one lane lower, same warp when outlet_fused)
         if (outlet_fused && x0 + 32 * warp <= L.nx - 1 && L.nx - 1 < x0 + 32 * warp + 32) {
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(32 * (C + 1), C == 8 ? 2 : 1) k_fused_tma(cons
 #pragma unroll
             for (int i = 0; i < Q; ++i) g[i] = __shfl_up_sync(0xffffffffu, f[i], 1);
             const uint32_t fm = __shfl_up_sync(0xffffffffu, fk, 1);
-            if (x == L.nx - 1 && !(fk & FLAG_SOLID) && !(fm & FLAG_SOLID)) nebb<false>(g, f, 0.f, L.rho_out);
+            if (x == L.nx - 1 && !(fk & FLAG_SOLID) && !(fm & FLAG_SOLID)) nebb(false, g, f, 0.f, L.rho_out);
         }
 
         if (inrow) {

@@ -44,11 +44,14 @@ namespace {
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 #include "fused_common.cuh"
+#include "collide2.cuh"
 #include "fused_reg.cuh"
 #include "fused_tma.cuh"
 #include "fused_async.cuh"
 #include "fused_split.cuh"
 #include "fused_half.cuh"
+#include "fused_cells.cuh"
+#include "fused_edge.cuh"
 #include "readouts.cuh"
 
 // Outlet/inlet rows on the pitched layout, for lattices whose x=nx-2 and x=nx-1 do not
@@ -68,8 +71,7 @@ __device__ __forceinline__ void bc_row(const lbm_lattice& L, T* __restrict__ fd,
         float g[Q], o[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) g[i] = ldpop(fd + (long long)i * L.cells + c1, i, inv_scale);
-        if (s == 0) nebb<true>(g, o, L.uin[j], L.rho_out);
-        else nebb<false>(g, o, 0.f, L.rho_out);
+        nebb(s == 0, g, o, s == 0 ? L.uin[j] : 0.f, L.rho_out);
 #pragma unroll
         for (int i = 0; i < Q; ++i) stpop(fd + (long long)i * L.cells + c0, i, o[i], scale);
     }
@@ -126,7 +128,7 @@ __global__ void __launch_bounds__(256) k_ref_step(const float* __restrict__ fs, 
     const float cf = cfw[c];
     if (wm && cf > 0.f) wall_function(f, wm, cf, ux[c], uy[c], uz[c], rho[c], uref[c]);
     float r, u, v, w;
-    collide(f, Fx[c], Fy[c], Fz[c], tau0, csmag2, r, u, v, w);
+    collide<true>(f, Fx[c], Fy[c], Fz[c], tau0, csmag2, r, u, v, w);
 #pragma unroll
     for (int i = 0; i < Q; ++i) fd[(long long)i * N + c] = f[i];
     rho[c] = r; ux[c] = u; uy[c] = v; uz[c] = w;
@@ -147,8 +149,7 @@ __global__ void k_ref_bc(float* __restrict__ fd, const uint8_t* __restrict__ sol
         float g[Q], o[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) g[i] = fd[(long long)i * N + c1];
-        if (s == 0) nebb<true>(g, o, uin[j], rho_out);
-        else nebb<false>(g, o, 0.f, rho_out);
+        nebb(s == 0, g, o, s == 0 ? uin[j] : 0.f, rho_out);
 #pragma unroll
         for (int i = 0; i < Q; ++i) fd[(long long)i * N + c0] = o[i];
     }
@@ -528,47 +529,40 @@ int launch_async(const lbm_lattice& L, const float* fs, float* fd, uint32_t mode
     }
 }
 
-template <int V, bool PLAIN, bool OUT, bool UCOL, bool AVG>
-int launch_rows_t(const lbm_lattice& L, const uint32_t* list, int n, const float* fs, float* fd, const lbm_tile& t,
-                  cudaStream_t st)
+// CTAs for `warps` warp passes: one pass per warp, or, with tile.ctas_per_sm set, that many
+// resident CTAs per SM striding over them.
+unsigned pass_grid(long long warps, const lbm_tile& t)
 {
-    if (n <= 0) return LBM_OK;
-    auto kern = k_rows<V, PLAIN, OUT, UCOL, AVG>;
-    const int threads = 32 * t.warps;
-    const int per_sm = occupancy(kern, threads, 0, t.ctas_per_sm);
-    long long grid = (long long)sm_count() * per_sm;
-    const long long need = ((long long)n + t.warps - 1) / t.warps;
-    if (grid > need) grid = need;
-    kern<<<(unsigned)grid, threads, 0, st>>>(L, pull_offsets(L), list, n, fs, fd);
-    return check_launch(PLAIN ? "k_rows<plain>" : "k_rows<special>");
+    const long long need = (warps + t.warps - 1) / t.warps, held = (long long)sm_count() * t.ctas_per_sm;
+    return (unsigned)(held > 0 && held < need ? held : need);
 }
 
-template <int V, int PASSES, bool OUT, bool AVG, typename T>
-int launch_edge(const lbm_lattice& L, const T* fs, T* fd, float scale, const lbm_tile& t, cudaStream_t st)
+template <int V, bool OUT, bool AVG>
+int launch_rows_t(const lbm_lattice& L, const float* fs, float* fd, const lbm_tile& t, cudaStream_t st)
 {
-    if (L.n_edge <= 0) return LBM_OK;
-    auto kern = k_rows_edge<V, PASSES, OUT, AVG, T>;
-    const int threads = 32 * t.warps;
-    const int per_sm = occupancy(kern, threads, 0, t.ctas_per_sm);
-    long long grid = (long long)sm_count() * per_sm;
-    const long long need = ((long long)L.n_edge + t.warps - 1) / t.warps;
-    if (grid > need) grid = need;
-    kern<<<(unsigned)grid, threads, 0, st>>>(L, pull_offsets(L), L.rows_edge, L.n_edge, fs, fd, scale);
-    return check_launch("k_rows_edge");
+    if (L.n_plain <= 0) return LBM_OK;
+    k_rows<V, OUT, AVG><<<pass_grid(L.n_plain, t), 32 * t.warps, 0, st>>>(L, pull_offsets(L), L.rows_plain, L.n_plain,
+                                                                          fs, fd);
+    return check_launch("k_rows");
 }
 
-template <int V, bool OUT, bool UCOL, bool AVG>
-int launch_general_f(const lbm_lattice& L, const float* fs, float* fd, const lbm_tile& t, cudaStream_t st)
+// Special list (k_cells) and edge list (k_edge), segments of 32*CPL cells.
+template <int CPL, bool OUT, bool UCOL, bool AVG, typename T>
+int launch_cells(const lbm_lattice& L, const T* fs, T* fd, float scale, const lbm_tile& t, cudaStream_t st)
 {
-    if (L.n_special <= 0) return LBM_OK;
-    auto kern = k_general<V, 1, OUT, UCOL, AVG, float>;
     const int threads = 32 * t.warps;
-    const int per_sm = occupancy(kern, threads, 0, t.ctas_per_sm);
-    long long grid = (long long)sm_count() * per_sm;
-    const long long need = ((long long)L.n_special + t.warps - 1) / t.warps;
-    if (grid > need) grid = need;
-    kern<<<(unsigned)grid, threads, 0, st>>>(L, pull_offsets(L), L.rows_special, L.n_special, fs, fd, 1.f);
-    return check_launch("k_general");
+    if (L.n_special > 0) {
+        k_cells<CPL, OUT, UCOL, AVG, T><<<pass_grid((long long)L.n_special * CPL, t), threads, 0, st>>>(
+            L, L.rows_special, L.n_special, fs, fd, scale);
+        if (int e = check_launch("k_cells")) return e;
+    }
+    if (L.n_edge > 0) {
+        const long long warps = CPL == 2 ? ((long long)L.n_edge + 1) / 2 : (long long)L.n_edge * (CPL / 4);
+        k_edge<CPL, OUT, AVG, T><<<pass_grid(warps, t), threads, 0, st>>>(L, pull_offsets(L), L.rows_edge, L.n_edge, fs,
+                                                                         fd, scale);
+        return check_launch("k_edge");
+    }
+    return LBM_OK;
 }
 
 template <int V, bool OUT, bool UCOL, bool AVG>
@@ -586,11 +580,8 @@ int launch_split_t(const lbm_lattice& L, const float* fs, float* fd, const lbm_t
         ts.ctas_per_sm = 0;
     }
     int e = LBM_OK;
-    if (!(mode & LBM_STEP_SKIP_PLAIN)) e = launch_rows_t<V, true, OUT, false, AVG>(L, L.rows_plain, L.n_plain, fs, fd, t, st);
-    if (!e && !(mode & LBM_STEP_SKIP_SPECIAL)) {
-        e = launch_edge<V, 1, OUT, AVG, float>(L, fs, fd, 1.f, ts, sst);
-        if (!e) e = launch_general_f<V, OUT, UCOL, AVG>(L, fs, fd, ts, sst);
-    }
+    if (!(mode & LBM_STEP_SKIP_PLAIN)) e = launch_rows_t<V, OUT, AVG>(L, fs, fd, t, st);
+    if (!e && !(mode & LBM_STEP_SKIP_SPECIAL)) e = launch_cells<V, OUT, UCOL, AVG, float>(L, fs, fd, 1.f, ts, sst);
     if (overlap) {
         const int ej = overlap_join(st, sst, lk);
         if (!e) e = ej;
@@ -637,29 +628,11 @@ int launch_tma(const lbm_lattice& L, const float* fs, float* fd, uint32_t mode, 
 // ---------------------------------------------------------------------------------------------
 // 16-bit storage launchers (fused_half.cuh)
 // ---------------------------------------------------------------------------------------------
-// warps_needed: warps that have work (default: one list entry per warp)
-template <typename K>
-int launch_list(K kern, const char* name, const lbm_lattice& L, const uint32_t* list, int n, const __half* hs,
-                __half* hd, float scale, const lbm_tile& t, cudaStream_t st, long long warps_needed = -1)
-{
-    if (n <= 0) return LBM_OK;
-    const int threads = 32 * t.warps;
-    const int per_sm = occupancy(kern, threads, 0, t.ctas_per_sm);
-    long long grid = (long long)sm_count() * per_sm;
-    if (warps_needed < 0) warps_needed = n;
-    const long long need = (warps_needed + t.warps - 1) / t.warps;
-    if (grid > need) grid = need;
-    kern<<<(unsigned)grid, threads, 0, st>>>(L, pull_offsets(L), list, n, hs, hd, scale);
-    return check_launch(name);
-}
-
-// CPL = cells_per_lane of the lists (segments of 32*CPL cells); the plain kernel runs 8 cells
-// per lane in groups of 4*CPL lanes, the edge and general paths VG cells per lane in PASSES passes.
+// CPL = cells_per_lane of the lists (segments of 32*CPL cells).
 template <int CPL, bool OUT, bool UCOL, bool AVG>
 int launch_split_h_t(const lbm_lattice& L, const __half* hs, __half* hd, float scale, const lbm_tile& t,
                      uint32_t mode, cudaStream_t st)
 {
-    constexpr int VG = CPL == 2 ? 2 : 4, PASSES = CPL / VG;
     // LBM_STEP_OVERLAP: edge and special kernels on the side stream beside the plain kernel, whose
     // CTAs per SM tile.ctas_per_sm then limits alone
     const bool overlap = (mode & LBM_STEP_OVERLAP) && !(mode & (LBM_STEP_SKIP_PLAIN | LBM_STEP_SKIP_SPECIAL));
@@ -672,31 +645,21 @@ int launch_split_h_t(const lbm_lattice& L, const __half* hs, __half* hd, float s
     }
     int err = LBM_OK;
     if (!(mode & LBM_STEP_SKIP_PLAIN) && L.n_plain > 0) {
-        // plain kernel: VP cells per lane (tile.stages 4 or 8; 0 = 8), 32*CPL/VP lanes per segment,
-        // so a warp takes VP/CPL list entries per pass
-        int e = LBM_OK;
-        bool done = false;
-        if constexpr (CPL <= 4) {
-            if (t.stages == 4) {
-                const long long warps = (L.n_plain + 4 / CPL - 1) / (4 / CPL);
-                e = launch_list(k_rows_h_plain<4, 8 * CPL, OUT, AVG>, "k_rows_h_plain", L, L.rows_plain, L.n_plain,
-                                hs, hd, scale, t, st, warps);
-                done = true;
-            }
+        // plain kernel: VP cells per lane (tile.stages 4 or 8; 0 = 4, or 8 on 256-cell segments),
+        // 32*CPL/VP lanes per segment, so a warp takes VP/CPL list entries per pass
+        const PullOffsets po = pull_offsets(L);
+        const int threads = 32 * t.warps;
+        if (CPL > 4 || t.stages == 8) {
+            const unsigned grid = pass_grid(((long long)L.n_plain + 8 / CPL - 1) / (8 / CPL), t);
+            k_rows_h_plain<8, 4 * CPL, OUT, AVG><<<grid, threads, 0, st>>>(L, po, L.rows_plain, L.n_plain, hs, hd, scale);
+        } else if constexpr (CPL <= 4) {
+            const unsigned grid = pass_grid(((long long)L.n_plain + 4 / CPL - 1) / (4 / CPL), t);
+            k_rows_h_plain<4, 8 * CPL, OUT, AVG><<<grid, threads, 0, st>>>(L, po, L.rows_plain, L.n_plain, hs, hd, scale);
         }
-        if (!done) {
-            const long long warps = (L.n_plain + 8 / CPL - 1) / (8 / CPL);
-            e = launch_list(k_rows_h_plain<8, 4 * CPL, OUT, AVG>, "k_rows_h_plain", L, L.rows_plain, L.n_plain, hs,
-                            hd, scale, t, st, warps);
-        }
-        err = e;
+        err = check_launch("k_rows_h_plain");
     }
-    if (!err && !(mode & LBM_STEP_SKIP_SPECIAL)) {
-        err = launch_edge<VG, PASSES, OUT, AVG, __half>(L, hs, hd, scale, ts, sst);
-        if (!err)
-            err = launch_list(k_general<VG, PASSES, OUT, UCOL, AVG, __half>, "k_general", L, L.rows_special,
-                              L.n_special, hs, hd, scale, ts, sst);
-    }
+    if (!err && !(mode & LBM_STEP_SKIP_SPECIAL))
+        err = launch_cells<CPL, OUT, UCOL, AVG, __half>(L, hs, hd, scale, ts, sst);
     if (overlap) {
         const int ej = overlap_join(st, sst, lk);
         if (!err) err = ej;
@@ -758,12 +721,7 @@ int launch_batch_list(K kern, const char* name, int n, long long warps_needed, c
                       Args... args)
 {
     if (n <= 0) return LBM_OK;
-    const int threads = 32 * t.warps;
-    const int per_sm = occupancy(kern, threads, 0, t.ctas_per_sm);
-    long long grid = (long long)sm_count() * per_sm;
-    const long long need = (warps_needed + t.warps - 1) / t.warps;
-    if (grid > need) grid = need;
-    kern<<<(unsigned)grid, threads, 0, st>>>(args...);
+    kern<<<pass_grid(warps_needed, t), 32 * t.warps, 0, st>>>(args...);
     return check_launch(name);
 }
 
@@ -773,20 +731,20 @@ int launch_batch_t(const lbm_batch& b, const BatchDesc& B, int parity, uint32_t 
 {
     if (!(mode & LBM_STEP_SKIP_PLAIN)) {
         int e;
-        if (t.stages == 4)
-            e = launch_batch_list(k_batch_plain<4, 16, OUT, AVG>, "k_batch_plain", b.n_plain, (b.n_plain + 1) / 2, t,
+        if (t.stages == 8)
+            e = launch_batch_list(k_batch_plain<8, 8, OUT, AVG>, "k_batch_plain", b.n_plain, (b.n_plain + 3LL) / 4, t,
                                   st, B, parity, b.rows_plain, b.n_plain);
         else
-            e = launch_batch_list(k_batch_plain<8, 8, OUT, AVG>, "k_batch_plain", b.n_plain, (b.n_plain + 3) / 4, t,
+            e = launch_batch_list(k_batch_plain<4, 16, OUT, AVG>, "k_batch_plain", b.n_plain, (b.n_plain + 1LL) / 2, t,
                                   st, B, parity, b.rows_plain, b.n_plain);
         if (e) return e;
     }
     if (mode & LBM_STEP_SKIP_SPECIAL) return LBM_OK;
-    if (int e = launch_batch_list(k_batch_edge<OUT, AVG>, "k_batch_edge", b.n_edge, b.n_edge, t, st, B, parity,
-                                  b.rows_edge, b.n_edge))
-        return e;
-    if (int e = launch_batch_list(k_batch_general<OUT, UCOL, AVG>, "k_batch_general", b.n_special, b.n_special, t, st,
+    if (int e = launch_batch_list(k_batch_cells<OUT, UCOL, AVG>, "k_batch_cells", b.n_special, 2LL * b.n_special, t, st,
                                   B, parity, b.rows_special, b.n_special))
+        return e;
+    if (int e = launch_batch_list(k_batch_edge<OUT, AVG>, "k_batch_edge", b.n_edge, (b.n_edge + 1LL) / 2, t, st, B,
+                                  parity, b.rows_edge, b.n_edge))
         return e;
     if (OUT && b.n_solid > 0) {
         long long grid = ((long long)b.n_solid * 32 + 127) / 128;
@@ -1277,8 +1235,8 @@ int lbm_fused_step_h(const lbm_lattice* lat, const uint16_t* hs, uint16_t* hd, f
     __half* d16 = reinterpret_cast<__half*>(hd);
     if (int e = launch_split_h(L, s16, d16, scale, mode, t, st)) return e;
     if (mode & LBM_STEP_SKIP_SPECIAL) return LBM_OK;
-    const int vg = cpl == 2 ? 2 : 4;
-    if ((L.nx - 1) % (32 * vg) == 0) {  // x=nx-2 and x=nx-1 in different segments: the outlet gets its own pass
+    const int join = 32 * (cpl == 2 ? 2 : 4);   // k_cells joins the outlet across passes inside this many cells
+    if ((L.nx - 1) % join == 0) {  // x=nx-2 and x=nx-1 in different segments: the outlet gets its own pass
         const long long M = (long long)L.ny * L.nz;
         k_bc_rows<__half><<<(unsigned)((M + 127) / 128), 128, 0, st>>>(L, d16, 2, scale);
         return check_launch("k_bc_rows");

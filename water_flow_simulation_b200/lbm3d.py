@@ -36,10 +36,10 @@ MIRZ = np.array([0, 1, 2, 3, 4, 6, 5, 7, 8, 9, 10, 13, 14, 11, 12, 17, 18, 15, 1
 
 AVG_FIELDS = ("ux", "uy", "uz", "rho", "sp", "uxx")
 # (pipeline, cells_per_lane, warps, stages, ctas_per_sm): work lists over 128-cell row segments,
-# 4 warps per CTA, as many CTAs per SM as fit
+# 4 warps per CTA, one segment per warp
 DEFAULT_TILE = (3, 4, 4, 0, 0)
-# 16-bit storage: work lists over 64-cell row segments (plain segments: 8 lanes of one 16-byte
-# vector of 8 cells each)
+# 16-bit storage: work lists over 64-cell row segments (plain segments: 16 lanes of one 8-byte
+# vector of 4 cells each)
 DEFAULT_TILE_FP16 = (3, 2, 4, 0, 0)
 STORAGES = ("fp32", "fp16")
 # |f_i - w_i| < 65504 / 2^14 ~ 4 is representable (populations of a stable lattice lie in (0, 1)),
