@@ -186,6 +186,12 @@ typedef struct lbm_tile {
 int lbm_build_flags(const lbm_lattice *lat, const uint8_t *solid, const uint8_t *bedwall,
                     uint32_t *flags, void *stream);
 
+/* Rows of nx elements of elem_bytes (1 or 4), contiguous, to rows of `pitch` elements (a multiple
+ * of 4) filled up with `pad` (its low byte for 1-byte elements): the layout of the per-cell
+ * arrays.  dst, and src for 4-byte elements, 4-byte aligned. */
+int lbm_pitch_rows(const void *src, void *dst, int elem_bytes, int nx, int pitch, int64_t rows, uint32_t pad,
+                   void *stream);
+
 /* 1D-profile start, floodsim/lbm3d.py:362-364 + 377-384: f = feq(rho=1,
  * u=(uin(y,z),0,0)) for fluid cells, feq(1,0) for solid and padding cells,
  * evaluated in float64 like the reference's NumPy code.  f: float[19*cells]. */

@@ -131,6 +131,7 @@ SIGNATURES = {
     "lbm_bc_f64": (I32, [P, P, P, I32, I32, I32, F64, P]),
     "lbm_update_uref_f64": (I32, [P] * 5 + [I32] * 3 + [P]),
     "lbm_build_flags": (I32, [ctypes.POINTER(Lattice), P, P, P, P]),
+    "lbm_pitch_rows": (I32, [P, P, I32, I32, I32, ctypes.c_int64, U32, P]),
     "lbm_init_equilibrium": (I32, [ctypes.POINTER(Lattice), P, P]),
     "lbm_fused_step": (I32, [ctypes.POINTER(Lattice), P, P, U32, ctypes.POINTER(Tile), P]),
     "lbm_build_worklists": (I32, [ctypes.POINTER(Lattice), I32, P, P, P, P, P, P, P]),

@@ -178,26 +178,6 @@ __global__ void __launch_bounds__(128, VP == 8 ? 3 : 5) k_rows_h_plain(const lbm
     }
 }
 
-// 16-bit start state: the float path's initial populations (k_init_equilibrium), stored as
-// scaled deviations.
-__global__ void k_init_equilibrium_h(const lbm_lattice L, __half* __restrict__ h, float scale)
-{
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= L.cells) return;
-    const int x = (int)(c % L.pitch), y = (int)((c / L.pitch) % L.ny), z = (int)(c / ((long long)L.pitch * L.ny));
-    const bool fluid = x < L.nx && !(L.flags[c] & FLAG_SOLID);
-    const float u = fluid ? L.uin[y + (long long)L.ny * z] : 0.f;
-    const double ud = (double)u;
-    const float q = __fmul_rn(__fmul_rn(1.5f, u), u);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        const double cu = __dmul_rn((double)(3 * cx(i)), ud);
-        const double poly = __dsub_rn(__dadd_rn(__dadd_rn(1.0, cu), __dmul_rn(__dmul_rn(0.5, cu), cu)), (double)q);
-        const float f = __double2float_rn(__dmul_rn(wgt64(i), poly));
-        h[(long long)i * L.cells + c] = __float2half_rn(__fmul_rn(__fsub_rn(f, wgt(i)), scale));
-    }
-}
-
 // float populations <-> 16-bit storage, n = 19*cells elements (direction i = element / cells).
 __global__ void k_pack_populations(const float* __restrict__ f, __half* __restrict__ h, long long cells, float scale)
 {

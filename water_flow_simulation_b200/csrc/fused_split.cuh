@@ -35,81 +35,6 @@ __device__ __forceinline__ void decode_row(uint32_t id, int nseg, int ny, int& s
     z = (int)(yz / (uint32_t)ny);
 }
 
-// 0 plain, 1 solid, 2 special, 3 edge (see the file comment); one thread per segment.
-__global__ void k_classify(const lbm_lattice L, int V, uint8_t* __restrict__ cls)
-{
-    const int SEG = 32 * V;
-    const int nseg = (L.pitch + SEG - 1) / SEG;
-    const long long n = (long long)nseg * L.ny * L.nz;
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const int seg = (int)(id % nseg);
-    const long long yz = id / nseg;
-    const int y = (int)(yz % L.ny), z = (int)(yz / L.ny);
-    const long long rowc = ((long long)z * L.ny + y) * L.pitch;
-    const int xa = seg * SEG, xb = min(xa + SEG, L.pitch);
-    bool all_solid = true, any_special = false;
-    for (int x = xa; x < xb; ++x) {
-        const uint32_t fk = L.flags[rowc + x];
-        all_solid &= (fk & FLAG_SOLID) != 0;
-        if (x < L.nx) any_special |= (fk & (FLAG_SOLID | FLAG_WALLS | FLAG_WALLFN | FLAG_FORCE)) != 0;
-    }
-    // open rows: clear of the y walls and the bed; the row under the lid counts (its -z movers
-    // read the own row's mirrored populations at constant offsets)
-    if (L.sponge_cols > 0 && xb > L.nx - L.sponge_cols) any_special = true;   // per-cell relaxation time
-    const bool interior_row = y >= 1 && y <= L.ny - 2 && z >= 1 && z <= L.nz - 1;
-    const bool clear_of_edges = seg > 0 && xa + SEG < L.nx;
-    int c = 2;
-    if (all_solid) c = 1;
-    else if (interior_row && !any_special) c = clear_of_edges ? 0 : 3;
-    cls[id] = (uint8_t)c;
-}
-
-// Ordered stream compaction of the four classes by one CTA (one-time set-up work).
-// counts[c] receives the number of segments of class c; lists[c] their ids in order.
-__global__ void __launch_bounds__(1024) k_compact(const uint8_t* __restrict__ cls, long long n,
-                                                  uint32_t* __restrict__ plain, uint32_t* __restrict__ solid,
-                                                  uint32_t* __restrict__ special, uint32_t* __restrict__ edge,
-                                                  int* __restrict__ counts)
-{
-    constexpr int NC = 4;
-    __shared__ int warp_tot[NC][32];
-    __shared__ int base[NC];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < NC) base[tid] = 0;
-    __syncthreads();
-    uint32_t* const lists[NC] = {plain, solid, special, edge};
-    for (long long start = 0; start < n; start += blockDim.x) {
-        const long long i = start + tid;
-        const int c = i < n ? cls[i] : NC;
-        int rank[NC], tot_before[NC];
-#pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            const unsigned m = __ballot_sync(0xffffffffu, c == k);
-            rank[k] = __popc(m & ((1u << lane) - 1u));
-            if (lane == 0) warp_tot[k][warp] = __popc(m);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            int acc = 0;
-            for (int w = 0; w < warp; ++w) acc += warp_tot[k][w];
-            tot_before[k] = acc;
-        }
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-            if (c == k) lists[k][base[k] + tot_before[k] + rank[k]] = (uint32_t)i;
-        __syncthreads();
-        if (tid < NC) {
-            int sum = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) sum += warp_tot[tid][w];
-            base[tid] += sum;
-        }
-        __syncthreads();
-    }
-    if (tid < NC) counts[tid] = base[tid];
-}
-
 // Streaming stores of the V cells' 19 populations.
 template <int I, int V>
 __device__ __forceinline__ void store_pop(float* p, const float (&f)[V][Q])

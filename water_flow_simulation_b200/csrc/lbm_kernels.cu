@@ -158,68 +158,7 @@ __global__ void k_ref_bc(float* __restrict__ fd, const uint8_t* __restrict__ sol
 // ---------------------------------------------------------------------------------------------
 // Set-up kernels
 // ---------------------------------------------------------------------------------------------
-template <int I>
-__device__ __forceinline__ void flag_dir(uint32_t& wm, const uint8_t* __restrict__ solid, const lbm_lattice& L,
-                                         int x, int y, int z)
-{
-    const int xs = x - cx(I), ys = y - cy(I);
-    int zs = z - cz(I);
-    if (xs < 0 || xs >= L.nx) return;
-    if (zs >= L.nz) zs = z;
-    bool wall = (ys < 0 || ys >= L.ny || zs < 0);
-    if (!wall) wall = solid[xs + (long long)L.pitch * (ys + (long long)L.ny * zs)] != 0;
-    if (wall) wm |= (1u << I);
-}
-template <int... Is>
-__device__ __forceinline__ void flag_all(std::integer_sequence<int, Is...>, uint32_t& wm,
-                                         const uint8_t* __restrict__ solid, const lbm_lattice& L, int x, int y, int z)
-{
-    (flag_dir<Is>(wm, solid, L, x, y, z), ...);
-}
-
-__global__ void k_build_flags(const lbm_lattice L, const uint8_t* __restrict__ solid,
-                              const uint8_t* __restrict__ bedwall, uint32_t* __restrict__ flags)
-{
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= L.cells) return;
-    const int x = (int)(c % L.pitch), y = (int)((c / L.pitch) % L.ny), z = (int)(c / ((long long)L.pitch * L.ny));
-    if (x >= L.nx) { flags[c] = FLAG_GHOST | FLAG_SOLID; return; }
-    if (solid[c]) { flags[c] = FLAG_SOLID; return; }
-    uint32_t wm = 0;
-    flag_all(std::make_integer_sequence<int, Q>{}, wm, solid, L, x, y, z);
-    uint32_t fw = wm;
-    if (L.Fx[c] != 0.f || L.Fy[c] != 0.f || L.Fz[c] != 0.f) fw |= FLAG_FORCE;
-    if (wm && L.cfw[c] > 0.f) {
-        int nwx = 0, nwy = 0, nwz = 0;
-        for (int i = 1; i < Q; ++i)
-            if (wm & (1u << i)) { nwx -= cx(i); nwy -= cy(i); nwz -= cz(i); }
-        const int ax = ((wm >> 1) & 1) + ((wm >> 2) & 1), ay = ((wm >> 3) & 1) + ((wm >> 4) & 1),
-                  az = ((wm >> 5) & 1) + ((wm >> 6) & 1);
-        if (nwx * nwx + nwy * nwy + nwz * nwz > 0 && ax * ax + ay * ay + az * az > 0) fw |= FLAG_WALLFN;
-    }
-    if (bedwall && bedwall[c]) fw |= FLAG_BEDWALL;
-    flags[c] = fw;
-}
-
-// f = feq(1, (u,0,0)) evaluated with the operation order and float64/float32 mix of the
-// reference's NumPy start (floodsim/lbm3d.py:377-384): cu = (3*c_x)*u and the quadratic
-// in float64, 1.5*u*u in float32, rounded once to float32 at the end.
-__global__ void k_init_equilibrium(const lbm_lattice L, float* __restrict__ f)
-{
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= L.cells) return;
-    const int x = (int)(c % L.pitch), y = (int)((c / L.pitch) % L.ny), z = (int)(c / ((long long)L.pitch * L.ny));
-    const bool fluid = x < L.nx && !(L.flags[c] & FLAG_SOLID);
-    const float u = fluid ? L.uin[y + (long long)L.ny * z] : 0.f;
-    const double ud = (double)u;
-    const float q = __fmul_rn(__fmul_rn(1.5f, u), u);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        const double cu = __dmul_rn((double)(3 * cx(i)), ud);
-        const double poly = __dsub_rn(__dadd_rn(__dadd_rn(1.0, cu), __dmul_rn(__dmul_rn(0.5, cu), cu)), (double)q);
-        f[(long long)i * L.cells + c] = __double2float_rn(__dmul_rn(__dmul_rn(wgt64(i), 1.0), poly));
-    }
-}
+#include "setup.cuh"
 
 // Start state from a coarse flow prediction (the learned warm start): per fluid cell, the
 // prediction (du, v, w, drho) of the cell's position, trilinear between coarse voxel centres
@@ -760,6 +699,33 @@ int launch_batch_t(const lbm_batch& b, const BatchDesc& B, int parity, uint32_t 
     return check_launch("k_batch_bc_rows");
 }
 
+// Start state of every cell (setup.cuh).
+template <typename T>
+int launch_start(const lbm_lattice& L, T* f, float scale, cudaStream_t st, const char* who)
+{
+    const long long rows = (long long)L.ny * L.nz;
+    if (reinterpret_cast<uintptr_t>(f) % (4 * sizeof(T)) == 0 && aligned16(L.flags)) {
+        k_start_rows<T><<<row_grid(rows, L.pitch), 128, 0, st>>>(L, f, scale);
+    } else {
+        k_start_cells<T><<<(unsigned)((L.cells + 255) / 256), 256, 0, st>>>(L, f, scale);
+    }
+    return check_launch(who);
+}
+
+// Class bytes and the four lists of n segments (setup.cuh).
+int launch_worklists(const lbm_lattice& L, int cells_per_lane, long long n, uint8_t* scratch, uint32_t* plain,
+                     uint32_t* solid, uint32_t* special, uint32_t* edge, int32_t* counts, cudaStream_t st)
+{
+    const int per_block = cells_per_lane == 2 ? 16 : 8;         // segments of 256 threads
+    k_classify<<<(unsigned)((n + per_block - 1) / per_block), 256, 0, st>>>(L, cells_per_lane, scratch);
+    if (int e = check_launch("k_classify")) return e;
+    // chunks of at least 2048 entries, a multiple of 16 each, over at most one CTA per SM
+    long long chunk = (n + sm_count() - 1) / sm_count();
+    chunk = ((chunk < 2048 ? 2048 : chunk) + 15) / 16 * 16;
+    k_compact<<<(unsigned)((n + chunk - 1) / chunk), 1024, 0, st>>>(scratch, n, chunk, plain, solid, special, edge, counts);
+    return check_launch("k_compact");
+}
+
 // Row chunks of the profile reduction (pass 1 runs nx x chunks threads).
 int profile_chunks(const lbm_lattice& L) { return L.ny * L.nz < 256 ? L.ny * L.nz : 256; }
 
@@ -891,8 +857,29 @@ int lbm_build_flags(const lbm_lattice* lat, const uint8_t* solid, const uint8_t*
     L.flags = flags;
     if (int e = check_lattice(&L)) return e;
     if (!solid || !L.Fx || !L.Fy || !L.Fz || !L.cfw) return fail(LBM_ERR_ARG, "lbm_build_flags: NULL array");
-    k_build_flags<<<(unsigned)((L.cells + 255) / 256), 256, 0, as_stream(stream)>>>(L, solid, bedwall, flags);
+    const auto at = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+    const bool vec = ((at(L.Fx) | at(L.Fy) | at(L.Fz) | at(L.cfw) | at(flags)) & 15) == 0 && ((at(solid) | at(bedwall)) & 3) == 0;
+    if (vec) k_build_flags4<<<row_grid((long long)L.ny * L.nz, L.pitch), 128, 0, as_stream(stream)>>>(L, solid, bedwall, flags);
+    else k_build_flags<<<(unsigned)((L.cells + 255) / 256), 256, 0, as_stream(stream)>>>(L, solid, bedwall, flags);
     return check_launch("lbm_build_flags");
+}
+
+int lbm_pitch_rows(const void* src, void* dst, int elem_bytes, int nx, int pitch, int64_t rows, uint32_t pad, void* stream)
+{
+    g_err[0] = 0;
+    if (!src || !dst) return fail(LBM_ERR_ARG, "lbm_pitch_rows: NULL array");
+    if ((elem_bytes != 1 && elem_bytes != 4) || nx < 1 || pitch < nx || (pitch & 3) || rows < 1)
+        return fail(LBM_ERR_ARG, "lbm_pitch_rows: %d-byte elements, rows of %d in %d (1 or 4 bytes, pitch >= nx and a "
+                                 "multiple of 4)", elem_bytes, nx, pitch);
+    if (((reinterpret_cast<uintptr_t>(dst) | (elem_bytes == 4 ? reinterpret_cast<uintptr_t>(src) : 0)) & 3) != 0)
+        return fail(LBM_ERR_ARG, "lbm_pitch_rows: arrays must be 4-byte aligned");
+    if (elem_bytes == 4)
+        k_pitch_rows<uint32_t><<<row_grid(rows, pitch), 128, 0, as_stream(stream)>>>(
+            static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), nx, pitch, rows, pad);
+    else
+        k_pitch_rows<uint8_t><<<row_grid(rows, pitch), 128, 0, as_stream(stream)>>>(
+            static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), nx, pitch, rows, (uint8_t)pad);
+    return check_launch("lbm_pitch_rows");
 }
 
 int lbm_init_equilibrium(const lbm_lattice* lat, float* f, void* stream)
@@ -900,8 +887,7 @@ int lbm_init_equilibrium(const lbm_lattice* lat, float* f, void* stream)
     g_err[0] = 0;
     if (int e = check_lattice(lat)) return e;
     if (!f) return fail(LBM_ERR_ARG, "lbm_init_equilibrium: NULL f");
-    k_init_equilibrium<<<(unsigned)((lat->cells + 255) / 256), 256, 0, as_stream(stream)>>>(*lat, f);
-    return check_launch("lbm_init_equilibrium");
+    return launch_start(*lat, f, 1.f, as_stream(stream), "lbm_init_equilibrium");
 }
 
 int lbm_build_worklists(const lbm_lattice* lat, int cells_per_lane, uint8_t* scratch, uint32_t* plain,
@@ -917,10 +903,7 @@ int lbm_build_worklists(const lbm_lattice* lat, int cells_per_lane, uint8_t* scr
     const long long n = (long long)((lat->pitch + seg - 1) / seg) * lat->ny * lat->nz;
     if (n > 0xffffffffLL) return fail(LBM_ERR_ARG, "lbm_build_worklists: too many segments for 32-bit ids");
     cudaStream_t st = as_stream(stream);
-    k_classify<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(*lat, cells_per_lane, scratch);
-    if (int e = check_launch("k_classify")) return e;
-    k_compact<<<1, 1024, 0, st>>>(scratch, n, plain, solid, special, edge, counts);
-    return check_launch("k_compact");
+    return launch_worklists(*lat, cells_per_lane, n, scratch, plain, solid, special, edge, counts, st);
 }
 
 int lbm_build_worklists_noalloc(const lbm_lattice* lat, int cells_per_lane, uint32_t* plain, uint32_t* solid,
@@ -942,10 +925,7 @@ int lbm_build_worklists_noalloc(const lbm_lattice* lat, int cells_per_lane, uint
     uint8_t* scratch = nullptr;
     if (int e = noalloc_scratch(&scratch)) return e;
     cudaStream_t st = as_stream(stream);
-    k_classify<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(*lat, cells_per_lane, scratch);
-    if (int e = check_launch("k_classify")) return e;
-    k_compact<<<1, 1024, 0, st>>>(scratch, n, plain, solid, special, edge, counts);
-    return check_launch("k_compact");
+    return launch_worklists(*lat, cells_per_lane, n, scratch, plain, solid, special, edge, counts, st);
 }
 
 int lbm_fused_step(const lbm_lattice* lat, const float* fs, float* fd, uint32_t mode, const lbm_tile* tile,
@@ -1172,9 +1152,7 @@ int lbm_init_equilibrium_h(const lbm_lattice* lat, uint16_t* h, float scale, voi
     if (int e = check_lattice(lat)) return e;
     if (int e = check_scale(scale, "lbm_init_equilibrium_h")) return e;
     if (!h) return fail(LBM_ERR_ARG, "lbm_init_equilibrium_h: NULL h");
-    k_init_equilibrium_h<<<(unsigned)((lat->cells + 255) / 256), 256, 0, as_stream(stream)>>>(
-        *lat, reinterpret_cast<__half*>(h), scale);
-    return check_launch("lbm_init_equilibrium_h");
+    return launch_start(*lat, reinterpret_cast<__half*>(h), scale, as_stream(stream), "lbm_init_equilibrium_h");
 }
 
 int lbm_pack_populations(const lbm_lattice* lat, const float* f, uint16_t* h, float scale, void* stream)

@@ -123,7 +123,7 @@ class LBM3D:
         self._uy = torch.zeros(self.cells, dtype=f32, device=d)
         self._uz = torch.zeros(self.cells, dtype=f32, device=d)
         self._colU = torch.zeros(self.ny * self.pitch, dtype=f32, device=d)
-        self._flags = torch.zeros(self.cells, dtype=torch.int32, device=d)
+        self._flags = torch.empty(self.cells, dtype=torch.int32, device=d)
         self._status = torch.zeros(4, dtype=torch.int32, device=d)
         self._avg = None
         self._body_scratch = None
@@ -133,13 +133,13 @@ class LBM3D:
         self.f2 = torch.empty(19 * self.cells, dtype=pop_dtype, device=d)
         self._flag_versions = None
         self._build_flags()
-        if storage == "fp16":
-            nat.check(self.lib.lbm_init_equilibrium_h(self._lattice_ref(), ctypes_ptr(self.f), self.store_scale,
-                                                      self._stream()), "lbm_init_equilibrium_h")
-        else:
-            nat.check(self.lib.lbm_init_equilibrium(self._lattice_ref(), ctypes_ptr(self.f), self._stream()),
-                      "lbm_init_equilibrium")
-        self.f2.copy_(self.f)
+        for f in (self.f, self.f2):        # written twice: a copy would read the first one back
+            if storage == "fp16":
+                nat.check(self.lib.lbm_init_equilibrium_h(self._lattice_ref(), ctypes_ptr(f), self.store_scale,
+                                                          self._stream()), "lbm_init_equilibrium_h")
+            else:
+                nat.check(self.lib.lbm_init_equilibrium(self._lattice_ref(), ctypes_ptr(f), self._stream()),
+                          "lbm_init_equilibrium")
 
     # ------------------------------------------------------------------ layout helpers
     def _pitched(self, a, dtype, pad=0):
@@ -149,12 +149,14 @@ class LBM3D:
         if isinstance(a, torch.Tensor):
             if a.numel() != self.N:
                 raise TypeError(f"LBM3D: array of size {a.numel()} does not match the lattice ({self.N} cells)")
-            t = a.to(self.device, non_blocking=True).reshape(self.nz, self.ny, self.nx).to(dtype)
-            if self.pitch != self.nx:
-                b = torch.full((self.nz, self.ny, self.pitch), pad, dtype=dtype, device=self.device)
-                b[..., :self.nx] = t
-                t = b
-            return t.reshape(-1).contiguous()
+            t = a.to(self.device, non_blocking=True).reshape(self.nz, self.ny, self.nx)
+            if self.pitch == self.nx:
+                return t.to(dtype).reshape(-1).contiguous()
+            t = (t.view(torch.uint8) if t.dtype == torch.bool and dtype == torch.uint8 else t.to(dtype)).contiguous()
+            b = torch.empty(self.cells, dtype=dtype, device=self.device)
+            nat.check(self.lib.lbm_pitch_rows(ctypes_ptr(t), ctypes_ptr(b), t.element_size(), self.nx, self.pitch,
+                                              self.ny * self.nz, pad, self._stream()), "lbm_pitch_rows")
+            return b
         a = np.asarray(a)
         if a.dtype == bool:
             a = a.astype(np.uint8)
