@@ -196,12 +196,12 @@ class SurrogateNet:
     def loss_and_grad(self, x, dims, target, mask):
         """Forward, masked MSE against target (V, 4) and backward; gradients are added to dW/db."""
         torch = self.torch
-        out = self.forward(x, dims)
         Z, Y, X = dims
         V = Z * Y * X
         target = target.to(self.device, torch.float32).contiguous()
         mask = mask.to(self.device, torch.float32).contiguous()
-        n = max(float(mask.sum()), 1.0)
+        n = max(float(mask.sum()), 1.0)     # read back before the forward pass is queued: it waits for nothing else
+        out = self.forward(x, dims)
         dout = torch.empty_like(out)
         loss = torch.zeros(1, device=self.device)
         nat.check(self.lib.lbm_nn_mse(out.data_ptr(), N_OUT, target.data_ptr(), N_PRED, mask.data_ptr(), V, 1.0 / n,
