@@ -377,10 +377,22 @@ int lbm_move_particles(const lbm_lattice *lat, double *P, int64_t n, float vel, 
 int lbm_gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int M, int N, int K, void *D, int ldd,
                   int epilogue, const float *bias, int *err, void *stream);
 
+/* 3x3x3 convolutions of channels-last bf16 grids on the tensor cores, without a column matrix (tap
+ * order and zero padding as below).  lbm_conv3_bf16: D[v][n] = epilogue(sum_t sum_c x[tap t of v][c]
+ * W[n][t*C + c] + bias[n]), C a multiple of 64, N of 8, epilogues 2, 3 and 4 of lbm_gemm_bf16; the
+ * same values as that GEMM on the column matrix.  lbm_conv3_back: its gradient to the input,
+ * dX[v][c] = sum_t (sum_o g[u][o] Wt[t*C + c][o]) over the (u, t) that read v, Wt the transposed
+ * weights (27*C x O), O a multiple of 8, C of 64.  Pointers 16-byte aligned; err as lbm_gemm_bf16's. */
+int lbm_conv3_bf16(const uint16_t *x, int C, int X, int Y, int Z, const uint16_t *W, int N, void *D, int epilogue,
+                   const float *bias, int *err, void *stream);
+int lbm_conv3_back(const uint16_t *g, int O, int X, int Y, int Z, const uint16_t *Wt, int C, float *dX, int *err,
+                   void *stream);
+
 /* Support kernels of the learned warm start's network (no counterpart in the reference).
  * Activations are channels-last bf16 (x[v*C + c], voxel v = x + X*(y + Y*z) of a (Z, Y, X)
  * grid); a 3x3x3 tap t = (dz+1)*9 + (dy+1)*3 + (dx+1), zero outside the grid.
  *   im2col     col[v][t*C + c] = x[tap t of v][c]                (C a multiple of 8)
+ *   im2col_t   colT[t*C + c][v] = x[tap t of v][c], zero for v up to Vp (C and Vp multiples of 8)
  *   col2im     dx[v][c] = sum of dcol[u][t*C + c] over the (u, t) that read v   (float)
  *   transpose  out[c][r] = in[r][c] (bf16, R rows -> Rp >= R columns, zero padded)
  *   act_grad   g = dy * (y > 0) (relu) or dy, as bf16; dbias[c] += column sums of g
@@ -390,6 +402,7 @@ int lbm_gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int M,
  *   mse        masked mean-square error of pred[v][0..nout) (row stride Cp): loss += and dpred
  *   adam       Adam step on float32 weights (bias-corrected, step >= 1), refreshing a bf16 copy */
 int lbm_nn_im2col(const uint16_t *x, int C, int X, int Y, int Z, uint16_t *col, void *stream);
+int lbm_nn_im2col_t(const uint16_t *x, int C, int X, int Y, int Z, int64_t Vp, uint16_t *colT, void *stream);
 int lbm_nn_col2im(const float *dcol, int C, int X, int Y, int Z, float *dx, void *stream);
 int lbm_nn_transpose(const uint16_t *in, int64_t R, int C, int64_t Rp, uint16_t *out, void *stream);
 int lbm_nn_act_grad(const float *dy, const uint16_t *y, int64_t V, int C, int relu, uint16_t *g, float *dbias,

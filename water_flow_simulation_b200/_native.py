@@ -148,6 +148,9 @@ SIGNATURES = {
     "lbm_gemm_bf16": (I32, [P, I32, P, I32, I32, I32, I32, P, I32, I32, P, P, P]),
     "lbm_lift_coarse": (I32, [ctypes.POINTER(Lattice), P, I32, I32, I32, I32, I32, F32, F32, P, P]),
     "lbm_nn_im2col": (I32, [P, I32, I32, I32, I32, P, P]),
+    "lbm_conv3_bf16": (I32, [P, I32, I32, I32, I32, P, I32, P, I32, P, P, P]),
+    "lbm_conv3_back": (I32, [P, I32, I32, I32, I32, P, I32, P, P, P]),
+    "lbm_nn_im2col_t": (I32, [P, I32, I32, I32, I32, ctypes.c_int64, P, P]),
     "lbm_nn_col2im": (I32, [P, I32, I32, I32, I32, P, P]),
     "lbm_nn_transpose": (I32, [P, ctypes.c_int64, I32, ctypes.c_int64, P, P]),
     "lbm_nn_act_grad": (I32, [P, P, ctypes.c_int64, I32, I32, P, P, P]),

@@ -3,8 +3,9 @@
 // The network is a small 3D convolutional encoder-decoder on a coarse copy of the lattice.
 // Every convolution, forward and backward, is a GEMM on 5th-generation tensor cores:
 //   D[M x N] = A[M x K] * B[N x K]^T      A, B bf16, both K-major; accumulation f32 in TMEM
-// fed by CUDA-core gather/scatter kernels (im2col, col2im, transposes, pooling) and finished
-// by fused epilogues (bias, ReLU, bf16 store).  Three GEMM kernels, chosen per call:
+// finished by fused epilogues (bias, ReLU, bf16 store).  k_conv_fwd and k_conv_back read the
+// grids in place (no column matrix); the weight gradients and the first layer (8 channels) go
+// through gather kernels (k_im2col, k_im2col_t, transposes) and three GEMM kernels, chosen per call:
 //   k_gemm_ws    products with >= 1024 rows and >= 128 columns: persistent, warp-specialised,
 //                TMA ring + MMA thread + epilogue warps, accumulator transposed in TMEM;
 //   k_gemm_tma   smaller products: one tile per CTA, TMA ring, MMA thread;
@@ -701,7 +702,7 @@ int launch_gemm_any(int bn, const __nv_bfloat16* A, int lda, const __nv_bfloat16
     int status = LBM_OK;
     // D += products with a long K and few tiles (the weight gradients: K is the voxels): narrow tiles,
     // for as many CTAs as there are, and a ring deep enough that the one chain of MMAs never waits
-    // for a load.  64 x 1728 weights over 12,288 voxels: 54 CTAs instead of 7, 88 -> 20 us.  Splitting
+    // for a load.  64 x 1728 weights over 12,288 voxels: 54 CTAs instead of 7, 88 -> 43 us a layer.  Splitting
     // K would be faster still, but moves the sums by more than 2e-5.
     if constexpr (EPI == EPI_F32_ADD) {
         const long long wide = (long long)((M + GM - 1) / GM) * ((N + bn - 1) / bn);
@@ -711,6 +712,394 @@ int launch_gemm_any(int bn, const __nv_bfloat16* A, int lda, const __nv_bfloat16
     }
     if (launch_gemm_ws<EPI>(A, lda, B, ldb, M, N, K, D, ldd, bias, err, st, &status)) return status;
     return launch_gemm_bn<EPI>(bn, A, lda, B, ldb, M, N, K, D, ldd, bias, err, st);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Convolutions without a column matrix.  A 3x3x3 convolution of a channels-last grid is the same
+// GEMM with A's rows read in place: the 128 rows of a tile are the voxels of a box of the grid, and
+// the K tile of tap t and channels c0.. is that box shifted by the tap, one tiled TMA load whose
+// coordinates outside the grid read zero.  K runs over taps, then channels, as the columns of
+// k_im2col do, so the accumulation and the results are those of the GEMM on the column matrix.
+// What bounds it: the 27 shifted reads of the grid now come from L2 instead of the column matrix's
+// write and read in HBM (415 MB each way for 64 channels on 120k voxels).  A prediction on 120k
+// voxels (10 x 80 x 150) takes 389 us instead of 1069, a gradient on 12k voxels 816 instead of 1099.
+// The input layer's 8 channels (16 bytes a voxel, an eighth of a K tile) keep the column matrix.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
+                                            uint32_t mbar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(mbar)
+        : "memory");
+}
+
+// Boxes of 128 voxels over an X x Y x Z grid: box sides (powers of two) and the boxes along each axis.
+struct ConvTiles {
+    int X, Y, Z, bx, by, bz, nx, ny, nz;
+};
+// Voxel coordinates of the first voxel of box `tile`.
+__device__ __forceinline__ void tile_origin(const ConvTiles& g, int tile, int& x, int& y, int& z)
+{
+    x = tile % g.nx * g.bx;
+    y = tile / g.nx % g.ny * g.by;
+    z = tile / (g.nx * g.ny) * g.bz;
+}
+// Voxel of row r of the box at (x, y, z), or -1 outside the grid.
+__device__ __forceinline__ long long tile_voxel(const ConvTiles& g, int x, int y, int z, int r)
+{
+    x += r % g.bx;
+    y += r / g.bx % g.by;
+    z += r / (g.bx * g.by);
+    return x < g.X && y < g.Y && z < g.Z ? x + (long long)g.X * (y + (long long)g.Y * z) : -1;
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t (&r)[16], uint32_t addr)
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+        "%14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// Forward: D[v][n] = epilogue(sum_t sum_c x[v + off_t][c] W[n][t*C + c] + bias[n]), C a multiple of
+// 64.  One box x BN channels per CTA (two CTAs per SM, so one's epilogue runs beside the other's
+// loads), one loading thread, one MMA thread, a ring of S stages; waits bounded as in k_gemm_tma.
+template <int BN, int EPI, int S>
+__global__ void __launch_bounds__(128, 2) k_conv_fwd(const __grid_constant__ CUtensorMap tmX,
+                                                     const __grid_constant__ CUtensorMap tmW, const ConvTiles g, int C,
+                                                     int N, void* __restrict__ D, const float* __restrict__ bias,
+                                                     int* __restrict__ err)
+{
+    static_assert(BN == 32 || BN == 64 || BN == 128, "TMEM allocation is a power of two >= 32");
+    constexpr uint32_t A_BYTES = GM * 128, B_BYTES = BN * 128, STAGE = A_BYTES + B_BYTES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full[S], empty[S], done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n0 = blockIdx.y * BN, per_tap = C / GK, nk = 27 * per_tap;
+    int x0, y0, z0;
+    tile_origin(g, blockIdx.x, x0, y0, z0);
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(smem_u32(&full[s]), 1);
+            mbar_init(smem_u32(&empty[s]), 1);
+        }
+        mbar_init(smem_u32(&done), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        failed = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(BN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    if (warp == 0 && lane == 0) {
+        int issued = 0;
+        for (int kt = 0; kt < nk; ++kt, ++issued) {
+            const int s = kt % S, round = kt / S;
+            if (kt >= S && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((round - 1) & 1))) {
+                atomicExch(err, 1);
+                failed = 1;
+                break;
+            }
+            if (*(volatile int*)&failed) break;
+            const int t = kt / per_tap, c0 = kt % per_tap * GK;
+            const uint32_t a = smem_u32(sm + (size_t)s * STAGE), fb = smem_u32(&full[s]);
+            mbar_expect_tx(fb, STAGE);
+            tma_load_4d(a, &tmX, c0, x0 + t % 3 - 1, y0 + t / 3 % 3 - 1, z0 + t / 9 - 1, fb);
+            tma_load_2d(a + A_BYTES, &tmW, kt * GK, n0, fb);
+        }
+        // the last copies must have landed before the block can leave
+        for (int kt = (issued > S ? issued - S : 0); kt < issued; ++kt)
+            mbar_wait(smem_u32(&full[kt % S]), (uint32_t)((kt / S) & 1));
+    } else if (warp == 1 && lane == 0) {
+        const uint32_t idesc = idesc_bf16(BN);
+        for (int kt = 0; kt < nk; ++kt) {
+            const int s = kt % S, round = kt / S;
+            if (!mbar_wait(smem_u32(&full[s]), (uint32_t)(round & 1)) || *(volatile int*)&failed) {
+                atomicExch(err, 1);
+                failed = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a = smem_u32(sm + (size_t)s * STAGE);
+#pragma unroll
+            for (int kk = 0; kk < GK / 16; ++kk)
+                mma_bf16(tmem, umma_desc(a + 32 * kk), umma_desc(a + A_BYTES + 32 * kk), idesc, (kt | kk) != 0);
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                         ::"r"(smem_u32(&empty[s]))
+                         : "memory");
+        }
+        // `done` completes once every MMA issued has, a failed run's too
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                     ::"r"(smem_u32(&done))
+                     : "memory");
+    }
+    __syncwarp();
+    const bool ok = mbar_wait(smem_u32(&done), 0u);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (__syncthreads_or(!ok || failed)) {
+        if (tid == 0) atomicExch(err, 1);
+    } else {
+        const long long v = tile_voxel(g, x0, y0, z0, warp * 32 + lane);
+        const int cols = N - n0 < BN ? N - n0 : BN;        // a multiple of 8
+#pragma unroll 1
+        for (int c0 = 0; c0 < cols; c0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(r, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0);
+#pragma unroll
+            for (int q = 0; q < 16; q += 8) {
+                if (v < 0 || c0 + q >= cols) continue;
+                float o[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    o[j] = __uint_as_float(r[q + j]) + bias[n0 + c0 + q + j];
+                    if constexpr (EPI == EPI_BF16_BIAS_RELU) o[j] = fmaxf(o[j], 0.f);
+                }
+                const size_t at = (size_t)v * N + n0 + c0 + q;
+                if constexpr (EPI == EPI_F32_BIAS) {
+                    float4* d = reinterpret_cast<float4*>(static_cast<float*>(D) + at);
+                    d[0] = make_float4(o[0], o[1], o[2], o[3]);
+                    d[1] = make_float4(o[4], o[5], o[6], o[7]);
+                } else {
+                    __nv_bfloat16 h[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16_rn(o[j]);
+                    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(D) + at) = *reinterpret_cast<uint4*>(h);
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+}
+
+// Backward to the input: dX[v][c] = sum_t (sum_o g[v - off_t][o] Wt[t*C + c][o]), Wt the transposed
+// weights (27*C x O).  The column-matrix form made dcol (float32, 27 C values per voxel) and gathered
+// it; here a tap's product stays in one of two TMEM buffers, and the epilogue warps add it, in the
+// order of the taps and in float32 as the gather did, to sums they keep in registers while the next
+// tap's product is made.  Voxels outside the grid read zero and add nothing.
+// Roles as in k_gemm_ws: warp 0 loads, warp 1 issues the MMAs, warps 2-5 add and store.
+constexpr int kBackN = 64, kBackStages = 6;
+
+__global__ void __launch_bounds__(kWsThreads, 1) k_conv_back(const __grid_constant__ CUtensorMap tmG,
+                                                             const __grid_constant__ CUtensorMap tmW, const ConvTiles g,
+                                                             int O, int C, float* __restrict__ dX, int* __restrict__ err)
+{
+    constexpr int S = kBackStages, BN = kBackN;
+    constexpr uint32_t A_BYTES = GM * 128, B_BYTES = BN * 128, STAGE = A_BYTES + B_BYTES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full[S], empty[S], acc_full[2], acc_empty[2], drain;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n0 = blockIdx.y * BN, per_tap = (O + GK - 1) / GK;
+    int x0, y0, z0;
+    tile_origin(g, blockIdx.x, x0, y0, z0);
+    if (tid == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(smem_u32(&full[s]), 1);
+            mbar_init(smem_u32(&empty[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&acc_full[b]), 1);
+            mbar_init(smem_u32(&acc_empty[b]), 4);
+        }
+        mbar_init(smem_u32(&drain), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        failed = 0;
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(2 * BN)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    volatile int* vfailed = &failed;
+    if (warp == 0) {
+        if (lane == 0) {
+            int it = 0;
+            for (int t = 0; t < 27 && !*vfailed; ++t) {
+                const int u = 26 - t;                      // v - off_t is v's neighbour through tap 26 - t
+                for (int q = 0; q < per_tap; ++q, ++it) {
+                    const int s = it % S, round = it / S;
+                    if (it >= S && !mbar_wait(smem_u32(&empty[s]), (uint32_t)((round - 1) & 1))) {
+                        atomicExch(err, 1);
+                        *vfailed = 1;
+                    }
+                    if (*vfailed) break;
+                    const uint32_t a = smem_u32(sm + (size_t)s * STAGE), fb = smem_u32(&full[s]);
+                    mbar_expect_tx(fb, STAGE);
+                    tma_load_4d(a, &tmG, q * GK, x0 + u % 3 - 1, y0 + u / 3 % 3 - 1, z0 + u / 9 - 1, fb);
+                    tma_load_2d(a + A_BYTES, &tmW, q * GK, t * C + n0, fb);
+                }
+            }
+            for (int j = (it > S ? it - S : 0); j < it; ++j) mbar_wait(smem_u32(&full[j % S]), (uint32_t)((j / S) & 1));
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = idesc_bf16(BN);
+            int it = 0;
+            for (int t = 0; t < 27 && !*vfailed; ++t) {
+                const int b = t & 1;
+                if (t >= 2 && !mbar_wait(smem_u32(&acc_empty[b]), (uint32_t)((t / 2 - 1) & 1))) {
+                    atomicExch(err, 1);
+                    *vfailed = 1;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                bool ok = true;
+                for (int q = 0; q < per_tap; ++q, ++it) {
+                    const int s = it % S;
+                    if (!mbar_wait(smem_u32(&full[s]), (uint32_t)((it / S) & 1)) || *vfailed) {
+                        atomicExch(err, 1);
+                        *vfailed = 1;
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a = smem_u32(sm + (size_t)s * STAGE);
+#pragma unroll
+                    for (int kk = 0; kk < GK / 16; ++kk)
+                        mma_bf16(tmem + b * BN, umma_desc(a + 32 * kk), umma_desc(a + A_BYTES + 32 * kk), idesc,
+                                 (q | kk) != 0);
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                                 ::"r"(smem_u32(&empty[s]))
+                                 : "memory");
+                }
+                if (!ok) break;
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                             ::"r"(smem_u32(&acc_full[b]))
+                             : "memory");
+            }
+            // every MMA this thread issued has completed once `drain` does
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                         ::"r"(smem_u32(&drain))
+                         : "memory");
+            mbar_wait(smem_u32(&drain), 0u);
+        }
+    } else {
+        const int quarter = warp & 3;                      // TMEM lanes 32 quarter .. + 31: the box's rows
+        float sum[BN];
+#pragma unroll
+        for (int j = 0; j < BN; ++j) sum[j] = 0.f;
+        bool good = true;
+        for (int t = 0; t < 27; ++t) {
+            const int b = t & 1;
+            const bool ready = mbar_wait(smem_u32(&acc_full[b]), (uint32_t)((t / 2) & 1));
+            if (__any_sync(0xffffffffu, !ready || *vfailed)) {
+                if (lane == 0) {
+                    atomicExch(err, 1);
+                    *vfailed = 1;
+                }
+                good = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int c0 = 0; c0 < BN; c0 += 16) {
+                uint32_t r[16];
+                tmem_ld16(r, tmem + b * BN + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[b])) : "memory");
+        }
+        const long long v = tile_voxel(g, x0, y0, z0, quarter * 32 + lane);
+        if (good && v >= 0) {
+            float* d = dX + (size_t)v * C + n0;
+#pragma unroll
+            for (int j = 0; j < BN; j += 4)
+                if (n0 + j < C) *reinterpret_cast<float4*>(d + j) = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+}
+
+// Tensor map of a channels-last grid (C channels, bf16), boxes of 64 channels x the tile's voxels,
+// 128-byte swizzle, zero outside.
+bool bf16_grid_map(CUtensorMap* map, const __nv_bfloat16* base, int C, const ConvTiles& g)
+{
+    PfnEncodeTiled enc = encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)g.X, (cuuint64_t)g.Y, (cuuint64_t)g.Z};
+    const cuuint64_t row = (cuuint64_t)C * 2;
+    const cuuint64_t strides[3] = {row, row * g.X, row * g.X * g.Y};
+    const cuuint32_t box[4] = {(cuuint32_t)GK, (cuuint32_t)g.bx, (cuuint32_t)g.by, (cuuint32_t)g.bz};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The box of 128 voxels that covers the grid with the fewest boxes; of equals the longest in x.
+ConvTiles conv_tiles(int X, int Y, int Z)
+{
+    ConvTiles best{};
+    long long fewest = -1;
+    for (int bx = 128; bx >= 1; bx /= 2)
+        for (int by = 128 / bx; by >= 1; by /= 2) {
+            const int bz = 128 / (bx * by);
+            const ConvTiles g{X, Y, Z, bx, by, bz, (X + bx - 1) / bx, (Y + by - 1) / by, (Z + bz - 1) / bz};
+            const long long n = (long long)g.nx * g.ny * g.nz;
+            if (fewest < 0 || n < fewest) {
+                fewest = n;
+                best = g;
+            }
+        }
+    return best;
+}
+
+template <int BN, int EPI>
+int launch_conv_bn(const __nv_bfloat16* x, int C, const ConvTiles& g, const __nv_bfloat16* W, int N, void* D,
+                   const float* bias, int* err, cudaStream_t st)
+{
+    constexpr int S = 4;
+    CUtensorMap tx, tw;
+    if (!bf16_grid_map(&tx, x, C, g) || !bf16_tile_map(&tw, W, N, 27 * C, 27 * C, BN))
+        return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: no tensor map for this grid");
+    auto kern = k_conv_fwd<BN, EPI, S>;
+    const int smem = S * (GM * 128 + BN * 128) + 1024;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: %d bytes of shared memory: %s", smem, cudaGetErrorString(cudaGetLastError()));
+    kern<<<dim3((unsigned)(g.nx * g.ny * g.nz), (unsigned)((N + BN - 1) / BN)), 128, smem, st>>>(tx, tw, g, C, N, D, bias, err);
+    return check_launch("k_conv_fwd");
+}
+
+// Channels per CTA: all of up to 64 (a box is then read once), in blocks of 64 beyond; of 32 where
+// the boxes alone would leave most SMs without one (small grids).
+template <int EPI>
+int launch_conv(const __nv_bfloat16* x, int C, const ConvTiles& g, const __nv_bfloat16* W, int N, void* D,
+                const float* bias, int* err, cudaStream_t st)
+{
+    const long long boxes = (long long)g.nx * g.ny * g.nz;
+    if (N <= 32 || boxes * ((N + 63) / 64) * 2 <= sm_count()) return launch_conv_bn<32, EPI>(x, C, g, W, N, D, bias, err, st);
+    return launch_conv_bn<64, EPI>(x, C, g, W, N, D, bias, err, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -742,6 +1131,37 @@ __global__ void k_im2col(const __nv_bfloat16* __restrict__ Xin, int C, int X, in
     uint4 val = make_uint4(0, 0, 0, 0);
     if (tap_src(t, x, y, z, X, Y, Z, s)) val = *reinterpret_cast<const uint4*>(Xin + s * C + 8 * q);
     *reinterpret_cast<uint4*>(col + (v * 27 + t) * C + 8 * q) = val;
+}
+
+// The transpose of the column matrix, colT[t*C + c][v] = X[neighbour t of v][c], zero for v in
+// [V, Vp): the weight gradients' operand, without the column matrix in between.  A block takes 64
+// voxels x up to 64 channels of one tap through shared memory; Vp a multiple of 8.
+__global__ void __launch_bounds__(256) k_im2col_t(const __nv_bfloat16* __restrict__ Xin, int C, int X, int Y, int Z,
+                                                  long long Vp, __nv_bfloat16* __restrict__ colT)
+{
+    __shared__ __nv_bfloat16 tile[64][66];                 // [channel][voxel]
+    const long long V = (long long)X * Y * Z, v0 = (long long)blockIdx.x * 64;
+    const int t = blockIdx.y, cb = blockIdx.z * 64, nc = C - cb < 64 ? C - cb : 64;
+    for (int e = threadIdx.x; e < 64 * (nc / 8); e += 256) {
+        const int k = e / (nc / 8), q = e % (nc / 8);
+        const long long v = v0 + k;
+        uint4 val = make_uint4(0, 0, 0, 0);
+        long long s;
+        if (v < V && tap_src(t, (int)(v % X), (int)((v / X) % Y), (int)(v / ((long long)X * Y)), X, Y, Z, s))
+            val = __ldg(reinterpret_cast<const uint4*>(Xin + s * C + cb + 8 * q));
+        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&val);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tile[8 * q + j][k] = h[j];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < 8 * nc; e += 256) {
+        const int c = e / 8, q = e % 8;
+        if (v0 + 8 * q >= Vp) continue;
+        __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) h[j] = tile[c][8 * q + j];
+        *reinterpret_cast<uint4*>(colT + ((long long)t * C + cb + c) * Vp + v0 + 8 * q) = *reinterpret_cast<uint4*>(h);
+    }
 }
 
 // dX[v][c] = sum_t dcol[u][t*C + c] over the voxels u whose tap t reads v (u = v - offset_t).
@@ -936,6 +1356,64 @@ int lbm_nn_im2col(const uint16_t* x, int C, int X, int Y, int Z, uint16_t* col, 
     k_im2col<<<blocks(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
         reinterpret_cast<const __nv_bfloat16*>(x), C, X, Y, Z, reinterpret_cast<__nv_bfloat16*>(col));
     return check_launch("k_im2col");
+}
+
+int lbm_nn_im2col_t(const uint16_t* x, int C, int X, int Y, int Z, int64_t Vp, uint16_t* colT, void* stream)
+{
+    g_err[0] = 0;
+    const long long V = (long long)X * Y * Z;
+    if (!x || !colT || C < 8 || C % 8 || X < 1 || Y < 1 || Z < 1 || Vp < V || Vp % 8)
+        return fail(LBM_ERR_ARG, "lbm_nn_im2col_t: bad arguments (channels and Vp multiples of 8, Vp >= voxels)");
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(colT)) & 15)
+        return fail(LBM_ERR_ARG, "lbm_nn_im2col_t: x and colT must be 16-byte aligned");
+    k_im2col_t<<<dim3(blocks(Vp, 64), 27, (unsigned)((C + 63) / 64)), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const __nv_bfloat16*>(x), C, X, Y, Z, Vp, reinterpret_cast<__nv_bfloat16*>(colT));
+    return check_launch("k_im2col_t");
+}
+
+int lbm_conv3_bf16(const uint16_t* x, int C, int X, int Y, int Z, const uint16_t* W, int N, void* D, int epilogue,
+                   const float* bias, int* err, void* stream)
+{
+    g_err[0] = 0;
+    if (!x || !W || !D || !bias || !err) return fail(LBM_ERR_ARG, "lbm_conv3_bf16: NULL pointer");
+    if (C < 64 || C % 64 || N < 8 || N % 8 || X < 1 || Y < 1 || Z < 1)
+        return fail(LBM_ERR_ARG, "lbm_conv3_bf16: %d -> %d channels on %dx%dx%d (inputs a multiple of 64, outputs of 8)", C, N,
+                    X, Y, Z);
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(D)) & 15)
+        return fail(LBM_ERR_ARG, "lbm_conv3_bf16: x, W and D must be 16-byte aligned");
+    const __nv_bfloat16* xb = reinterpret_cast<const __nv_bfloat16*>(x);
+    const __nv_bfloat16* wb = reinterpret_cast<const __nv_bfloat16*>(W);
+    const ConvTiles g = conv_tiles(X, Y, Z);
+    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    switch (epilogue) {
+    case EPI_BF16_BIAS: return launch_conv<EPI_BF16_BIAS>(xb, C, g, wb, N, D, bias, err, st);
+    case EPI_BF16_BIAS_RELU: return launch_conv<EPI_BF16_BIAS_RELU>(xb, C, g, wb, N, D, bias, err, st);
+    case EPI_F32_BIAS: return launch_conv<EPI_F32_BIAS>(xb, C, g, wb, N, D, bias, err, st);
+    default: return fail(LBM_ERR_ARG, "lbm_conv3_bf16: epilogue %d (2, 3 or 4)", epilogue);
+    }
+}
+
+int lbm_conv3_back(const uint16_t* g, int O, int X, int Y, int Z, const uint16_t* Wt, int C, float* dX, int* err,
+                   void* stream)
+{
+    g_err[0] = 0;
+    if (!g || !Wt || !dX || !err) return fail(LBM_ERR_ARG, "lbm_conv3_back: NULL pointer");
+    if (O < 8 || O % 8 || C < 64 || C % 64 || X < 1 || Y < 1 || Z < 1)
+        return fail(LBM_ERR_ARG, "lbm_conv3_back: %d -> %d channels on %dx%dx%d (outputs a multiple of 8, inputs of 64)", O, C,
+                    X, Y, Z);
+    if ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(dX)) & 15)
+        return fail(LBM_ERR_ARG, "lbm_conv3_back: g, Wt and dX must be 16-byte aligned");
+    const ConvTiles t = conv_tiles(X, Y, Z);
+    CUtensorMap tg, tw;
+    if (!bf16_grid_map(&tg, reinterpret_cast<const __nv_bfloat16*>(g), O, t) ||
+        !bf16_tile_map(&tw, reinterpret_cast<const __nv_bfloat16*>(Wt), 27 * C, O, O, kBackN))
+        return fail(LBM_ERR_CUDA, "lbm_conv3_back: no tensor map for this grid");
+    const int smem = kBackStages * (GM * 128 + kBackN * 128) + 1024;
+    if (cudaFuncSetAttribute(k_conv_back, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        return fail(LBM_ERR_CUDA, "lbm_conv3_back: %d bytes of shared memory: %s", smem, cudaGetErrorString(cudaGetLastError()));
+    k_conv_back<<<dim3((unsigned)(t.nx * t.ny * t.nz), (unsigned)(C / kBackN)), kWsThreads, smem,
+                  reinterpret_cast<cudaStream_t>(stream)>>>(tg, tw, t, O, C, dX, err);
+    return check_launch("k_conv_back");
 }
 
 int lbm_nn_col2im(const float* dcol, int C, int X, int Y, int Z, float* dx, void* stream)

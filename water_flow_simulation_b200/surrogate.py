@@ -8,7 +8,8 @@ equilibrium populations and fields of a new start state (LBM3D.load_populations)
 the unmodified LBM runs on.
 
 Network (about 1.0M parameters, bf16 weights, float32 accumulation; every convolution,
-forward and backward, is a GEMM on the tensor cores, lbm_gemm_bf16):
+forward and backward, is a product on the tensor cores: lbm_conv3_bf16, lbm_conv3_back,
+lbm_gemm_bf16):
     a1 = relu(conv3 8->64 x)                      full coarse grid
     p  = pool2(a1)                                half grid
     a4 = relu(conv3 128->64 relu(conv3 128->128 relu(conv3 64->128 p)))
@@ -133,16 +134,17 @@ class SurrogateNet:
         _, cin, cout, relu = next(l for l in LAYERS if l[0] == name)
         Z, Y, X = dims
         V = Z * Y * X
-        col = torch.empty(V, 27 * cin, dtype=torch.bfloat16, device=self.device)
-        nat.check(self.lib.lbm_nn_im2col(x.data_ptr(), cin, X, Y, Z, col.data_ptr(), self._st()), "lbm_nn_im2col")
         P = self.p[name]
-        if f32_out:
-            y = torch.empty(V, cout, dtype=torch.float32, device=self.device)
-            self._gemm(col, 27 * cin, P["Wb"], 27 * cin, V, cout, 27 * cin, y, cout, 4, P["b"])
-        else:
-            y = torch.empty(V, cout, dtype=torch.bfloat16, device=self.device)
-            self._gemm(col, 27 * cin, P["Wb"], 27 * cin, V, cout, 27 * cin, y, cout, 3 if relu else 2, P["b"])
-        self.cache[name] = (col, y, dims, cin, cout, relu)
+        y = torch.empty(V, cout, dtype=torch.float32 if f32_out else torch.bfloat16, device=self.device)
+        epi = 4 if f32_out else 3 if relu else 2
+        if cin % 64 == 0:
+            nat.check(self.lib.lbm_conv3_bf16(x.data_ptr(), cin, X, Y, Z, P["Wb"].data_ptr(), cout, y.data_ptr(), epi,
+                                              P["b"].data_ptr(), self.err.data_ptr(), self._st()), "lbm_conv3_bf16")
+        else:                               # the input layer's 8 channels: through a column matrix
+            col = torch.empty(V, 27 * cin, dtype=torch.bfloat16, device=self.device)
+            nat.check(self.lib.lbm_nn_im2col(x.data_ptr(), cin, X, Y, Z, col.data_ptr(), self._st()), "lbm_nn_im2col")
+            self._gemm(col, 27 * cin, P["Wb"], 27 * cin, V, cout, 27 * cin, y, cout, epi, P["b"])
+        self.cache[name] = (x, y, dims, cin, cout, relu)
         return y
 
     def forward(self, x, dims):
@@ -163,7 +165,7 @@ class SurrogateNet:
     # ------------------------------------------------------------------ backward
     def _conv_back(self, name, dy, need_dx=True):
         torch = self.torch
-        col, y, dims, cin, cout, relu = self.cache[name]
+        x, y, dims, cin, cout, relu = self.cache[name]
         Z, Y, X = dims
         V = Z * Y * X
         Vp = _r8(V)
@@ -175,17 +177,16 @@ class SurrogateNet:
         gT = torch.empty(cout, Vp, dtype=torch.bfloat16, device=self.device)
         colT = torch.empty(27 * cin, Vp, dtype=torch.bfloat16, device=self.device)
         nat.check(self.lib.lbm_nn_transpose(g.data_ptr(), V, cout, Vp, gT.data_ptr(), st), "lbm_nn_transpose")
-        nat.check(self.lib.lbm_nn_transpose(col.data_ptr(), V, 27 * cin, Vp, colT.data_ptr(), st), "lbm_nn_transpose")
+        nat.check(self.lib.lbm_nn_im2col_t(x.data_ptr(), cin, X, Y, Z, Vp, colT.data_ptr(), st), "lbm_nn_im2col_t")
         self._gemm(gT, Vp, colT, Vp, cout, 27 * cin, Vp, P["dW"], 27 * cin, 1)          # dW += g^T col
         if not need_dx:
             return None
         Wt = torch.empty(27 * cin, cout, dtype=torch.bfloat16, device=self.device)
         nat.check(self.lib.lbm_nn_transpose(P["Wb"].data_ptr(), cout, 27 * cin, cout, Wt.data_ptr(), st),
                   "lbm_nn_transpose")
-        dcol = torch.empty(V, 27 * cin, dtype=torch.float32, device=self.device)
-        self._gemm(g, cout, Wt, cout, V, 27 * cin, cout, dcol, 27 * cin, 0)             # dcol = g W
         dx = torch.empty(V, cin, dtype=torch.float32, device=self.device)
-        nat.check(self.lib.lbm_nn_col2im(dcol.data_ptr(), cin, X, Y, Z, dx.data_ptr(), st), "lbm_nn_col2im")
+        nat.check(self.lib.lbm_conv3_back(g.data_ptr(), cout, X, Y, Z, Wt.data_ptr(), cin, dx.data_ptr(),
+                                          self.err.data_ptr(), st), "lbm_conv3_back")
         return dx
 
     def zero_grad(self):
