@@ -472,8 +472,10 @@ def run_b200(args, rank, world, local_rank):
     main = measure(args.storage, steps, None if args.quick else clocks)
     ms_max = main["ms"]
     counts = main["counts"]
-    # per step: plain, edge and special kernels; per output step also solid fields and column means
-    launches = steps * 3 + (steps // CHUNK) * 2 if counts else steps
+    # a step is one launch over the lists, or, held down, overlapped or with 8 cells per lane, plain,
+    # edge and special kernels; an output step is always these, then solid fields and column means
+    one = counts and main["V"] <= 4 and main["tile"][3] != 8 and not any(main["tile"][4:])
+    launches = steps * (1 if one else 3) + (steps // CHUNK) * (4 if one else 2) if counts else steps
     gemm = None
     if rank == 0 and not args.quick:   # the learned warm start's tensor-core GEMM (bf16, float32 accumulation)
         try:
@@ -689,7 +691,8 @@ def run_ensemble(args, rank, world, local_rank):
                               "batching_gain_over_fp16_single": single16_hours / chosen_hours},
            "fp16_single_glups_same_cases": single16_glups,
            "plain_fp32_ms_per_step": plain, "fp16_single_ms_per_step": single16,
-           "gpu_launches": (steps // BCHUNK) if tile == "persistent" else steps * 3 + (steps // BCHUNK) * 3,
+           "gpu_launches": (steps // BCHUNK) if tile == "persistent" else
+           steps * 4 + (steps // BCHUNK) * 2 if tile[3] == 8 or tile[4] else steps * 2 + (steps // BCHUNK) * 4,
            "clocks": clocks.summary(), "status_words": status}
     print(json.dumps(out), flush=True)
     return 0

@@ -4,9 +4,9 @@
 // A batch holds K lattices (boat cases of any sizes) in device memory: their lattice
 // descriptors, pull-offset tables, 16-bit storage scales and both population buffers of each.
 // Work-list entries carry the case in their top 8 bits and the row-segment id (of that case's
-// own 64-cell segments, cells_per_lane 2) in the low 24.  One step of the whole batch is then
-// a plain launch and one for the special and edge cells over the concatenated lists (plus the
-// solid-field, column-mean and outlet passes on output steps), whatever the sizes of the cases: small
+// own 64-cell segments, cells_per_lane 2) in the low 24.  One step of the whole batch is then one
+// launch over the concatenated lists and one for the outlet rows (output steps: a launch per list, and
+// the solid-field and column-mean passes), whatever the sizes of the cases: small
 // cases no longer leave the GPU idle between launches or in short tails, and the launch
 // count of a step does not grow with the number of cases.  Population buffers alternate by
 // step parity, so a chunk of an even number of steps can be captured once as a CUDA graph
@@ -120,6 +120,32 @@ __global__ void __launch_bounds__(128, 4) k_batch_edge(const BatchDesc B, int pa
     const long long W = ((long long)gridDim.x * blockDim.x) >> 5;
     for (long long b = 2 * (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < n_edge; b += 2 * W)
         batch_edge_pass<OUT, AVG, __half>(B, parity, edge, b, n_edge, lane);
+}
+
+// The three lists of a step in one launch (as k_all_lists): special passes, edge passes, plain passes.
+// Five cases of 1.7M cells: 134 us a step against 145 in three launches (137 at 4 CTAs per SM).
+template <bool UCOL>
+__global__ void __launch_bounds__(128, 5) k_batch_all(const BatchDesc B, int parity, const lbm_batch b)
+{
+    const int lane = threadIdx.x & 31;
+    int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (t < 2 * b.n_special) {
+        batch_cell_pass<false, UCOL, false, __half>(B, parity, __ldg(b.rows_special + (t >> 1)), t & 1, lane);
+        return;
+    }
+    t -= 2 * b.n_special;
+    if (2 * t < b.n_edge) {
+        batch_edge_pass<false, false, __half>(B, parity, b.rows_edge, 2LL * t, b.n_edge, lane);
+        return;
+    }
+    t -= (b.n_edge + 1) / 2;
+    const int p = 2 * t, grp = lane >> 4;
+    if (p < b.n_plain) {
+        const bool valid = p + grp < b.n_plain;
+        const BatchItem it = batch_item(B, parity, __ldg(b.rows_plain + (valid ? p + grp : p)));
+        h_plain_segment<4, 16, false, false>(B.lat[it.c], B.po[it.c], it.fs, it.fd, __ldg(B.scale + it.c), it.id,
+                                             lane & 15, valid);
+    }
 }
 
 template <bool AVG>

@@ -187,24 +187,30 @@ __device__ __forceinline__ void edge_lane(const lbm_lattice& L, const PullOffset
     }
 }
 
-// Edge list: entries are segments of 32*CPL cells; a warp pass takes PER_WARP entries of 64 cells
+// Edge list: entries are segments of 32*CPL cells; a warp pass takes two entries of 64 cells
 // each, one of 128, or half of one of 256.
+__host__ __device__ constexpr int edge_passes(int cpl, int nlist) { return cpl == 2 ? (nlist + 1) / 2 : nlist * (cpl / 4); }
+
+template <int CPL, bool OUT, bool AVG, typename T>
+__device__ __forceinline__ void edge_pass(const lbm_lattice& L, const PullOffsets& po, const uint32_t* __restrict__ list,
+                                          int nlist, const T* __restrict__ fs, T* __restrict__ fd, float scale, int t,
+                                          int lane)
+{
+    constexpr int G = CPL == 2 ? 16 : 32, PER_WARP = 32 / G, SEG = 32 * CPL, PASSES = SEG / (4 * G);
+    const int gl = lane % G, grp = lane / G, b = t / PASSES * PER_WARP;
+    const bool valid = b + grp < nlist;
+    int seg, y, z;
+    decode_row(__ldg(list + (valid ? b + grp : b)), (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
+    const int x0 = seg * SEG + t % PASSES * 4 * G + gl * 4;
+    edge_lane<G, OUT, AVG, T>(L, po, fs, fd, scale, 1.0f / scale, x0, y, z, gl, valid);
+}
+
 template <int CPL, bool OUT, bool AVG, typename T>
 __global__ void __launch_bounds__(128, std::is_same<T, float>::value ? 3 : 4)
     k_edge(const lbm_lattice L, const PullOffsets po, const uint32_t* __restrict__ list, int nlist,
            const T* __restrict__ fs, T* __restrict__ fd, float scale)
 {
-    constexpr int G = CPL == 2 ? 16 : 32, PER_WARP = 32 / G, SEG = 32 * CPL, PASSES = SEG / (4 * G);
-    const int lane = threadIdx.x & 31, gl = lane % G, grp = lane / G;
-    const long long W = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long total = ((long long)nlist + PER_WARP - 1) / PER_WARP * PASSES;
-    const int nseg = (L.pitch + SEG - 1) / SEG;
-    for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < total; t += W) {
-        const long long b = t / PASSES * PER_WARP;
-        const bool valid = b + grp < nlist;
-        int seg, y, z;
-        decode_row(__ldg(list + (valid ? b + grp : b)), nseg, L.ny, seg, y, z);
-        const int x0 = seg * SEG + (int)(t % PASSES) * 4 * G + gl * 4;
-        edge_lane<G, OUT, AVG, T>(L, po, fs, fd, scale, 1.0f / scale, x0, y, z, gl, valid);
-    }
+    const int lane = threadIdx.x & 31, W = (int)((gridDim.x * blockDim.x) >> 5), total = edge_passes(CPL, nlist);
+    for (int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); t < total; t += W)
+        edge_pass<CPL, OUT, AVG, T>(L, po, list, nlist, fs, fd, scale, t, lane);
 }

@@ -11,7 +11,8 @@
 //              and possibly padding: the first and last segment of an open row;
 //   solid   -- every cell solid (or padding);
 //   special -- everything else (walls, bed, lid, banks, hulls, forcing).
-// A step then runs
+// A step then runs k_all_lists (fused_all.cuh), the passes of the three moving lists in one launch;
+// an output step, an overlapped one or one with its grid held down runs a kernel per list:
 //   k_rows          over the plain list: 19 V-wide pulls at constant offsets (the +-1 x
 //                   neighbours by warp shuffle), collision with no force, 19 V-wide
 //                   streaming stores -- no flag word is read; this is where the cells are;
@@ -92,6 +93,39 @@ __device__ __forceinline__ float sponge_tau0(const lbm_lattice& L, int x)
     return __fadd_rn(L.tau0, __fmul_rn(__fsub_rn(L.sponge_tau, L.tau0), __fmul_rn(s, s)));
 }
 
+// One plain segment of 32*V cells (row-segment id `id`), V cells per lane.
+template <int V, bool OUT, bool AVG>
+__device__ __forceinline__ void plain_segment(const lbm_lattice& L, const PullOffsets& po, const float* __restrict__ fs,
+                                              float* __restrict__ fd, uint32_t id, int lane)
+{
+    constexpr int SEG = 32 * V;
+    int seg, y, z;
+    decode_row(id, (L.pitch + SEG - 1) / SEG, L.ny, seg, y, z);
+    const long long own = ((long long)z * L.ny + y) * L.pitch + seg * SEG + lane * V;
+    float f[V][Q];
+    float R[V], UX[V], UY[V], UZ[V];
+    pull_fast_all<V>(std::make_integer_sequence<int, Q>{}, f, fs + own, po, lane, z == L.nz - 1);
+#pragma unroll
+    for (int k = 0; k < V; k += 2) {
+        float2 d[Q], r2, ux2, uy2, uz2;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) d[i] = make_float2(f[k][i], f[k + 1][i]);
+        collide2<false, AVG>(d, 1.f, 1.f, L.tau0, L.csmag2, r2, ux2, uy2, uz2);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) { f[k][i] = d[i].x; f[k + 1][i] = d[i].y; }
+        R[k] = r2.x; UX[k] = ux2.x; UY[k] = uy2.x; UZ[k] = uz2.x;
+        R[k + 1] = r2.y; UX[k + 1] = ux2.y; UY[k + 1] = uy2.y; UZ[k + 1] = uz2.y;
+    }
+    store_pops<V>(std::make_integer_sequence<int, Q>{}, fd, L.cells, own, f);
+    if constexpr (OUT) {
+        store_fields<V, AVG>(L, own, R, UX, UY, UZ);
+        bool bad = false;
+#pragma unroll
+        for (int k = 0; k < V; ++k) bad |= !(R[k] > 0.f && R[k] < 3.4e38f);
+        if (bad) atomicOr(L.status, 1);
+    }
+}
+
 // Plain list: a warp pass per segment of 32*V cells, one pass per warp unless the grid is held
 // down (lbm_tile.ctas_per_sm).  Bound by HBM: with V = 4, 16 warps per SM (118 registers) and all
 // of a pass's 19 16-byte loads issued before anything waits, 155 KB are in flight per SM, and CTAs
@@ -102,38 +136,9 @@ __global__ void __launch_bounds__(128, V == 4 ? 4 : 6) k_rows(const lbm_lattice 
                                                               const uint32_t* __restrict__ list, int nlist,
                                                               const float* __restrict__ fs, float* __restrict__ fd)
 {
-    constexpr int SEG = 32 * V;
     const int lane = threadIdx.x & 31;
     const int gw = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), W = (int)((gridDim.x * blockDim.x) >> 5);
-    const int nseg = (L.pitch + SEG - 1) / SEG;
-    const long long S = L.cells;
-    for (int w = gw; w < nlist; w += W) {
-        int seg, y, z;
-        decode_row(__ldg(list + w), nseg, L.ny, seg, y, z);
-        const long long own = ((long long)z * L.ny + y) * L.pitch + seg * SEG + lane * V;
-        float f[V][Q];
-        float R[V], UX[V], UY[V], UZ[V];
-        pull_fast_all<V>(std::make_integer_sequence<int, Q>{}, f, fs + own, po, lane, z == L.nz - 1);
-#pragma unroll
-        for (int k = 0; k < V; k += 2) {
-            float2 d[Q], r2, ux2, uy2, uz2;
-#pragma unroll
-            for (int i = 0; i < Q; ++i) d[i] = make_float2(f[k][i], f[k + 1][i]);
-            collide2<false, AVG>(d, 1.f, 1.f, L.tau0, L.csmag2, r2, ux2, uy2, uz2);
-#pragma unroll
-            for (int i = 0; i < Q; ++i) { f[k][i] = d[i].x; f[k + 1][i] = d[i].y; }
-            R[k] = r2.x; UX[k] = ux2.x; UY[k] = uy2.x; UZ[k] = uz2.x;
-            R[k + 1] = r2.y; UX[k + 1] = ux2.y; UY[k + 1] = uy2.y; UZ[k + 1] = uz2.y;
-        }
-        store_pops<V>(std::make_integer_sequence<int, Q>{}, fd, S, own, f);
-        if constexpr (OUT) {
-            store_fields<V, AVG>(L, own, R, UX, UY, UZ);
-            bool bad = false;
-#pragma unroll
-            for (int k = 0; k < V; ++k) bad |= !(R[k] > 0.f && R[k] < 3.4e38f);
-            if (bad) atomicOr(L.status, 1);
-        }
-    }
+    for (int w = gw; w < nlist; w += W) plain_segment<V, OUT, AVG>(L, po, fs, fd, __ldg(list + w), lane);
 }
 
 // Output step: fields of one solid segment's V cells per lane (rho = 1, u = 0) and their

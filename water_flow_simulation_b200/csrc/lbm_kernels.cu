@@ -52,6 +52,7 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 #include "fused_half.cuh"
 #include "fused_cells.cuh"
 #include "fused_edge.cuh"
+#include "fused_all.cuh"
 #include "readouts.cuh"
 
 // Outlet/inlet rows on the pitched layout, for lattices whose x=nx-2 and x=nx-1 do not
@@ -496,18 +497,42 @@ int launch_cells(const lbm_lattice& L, const T* fs, T* fd, float scale, const lb
         if (int e = check_launch("k_cells")) return e;
     }
     if (L.n_edge > 0) {
-        const long long warps = CPL == 2 ? ((long long)L.n_edge + 1) / 2 : (long long)L.n_edge * (CPL / 4);
-        k_edge<CPL, OUT, AVG, T><<<pass_grid(warps, t), threads, 0, st>>>(L, pull_offsets(L), L.rows_edge, L.n_edge, fs,
-                                                                         fd, scale);
+        k_edge<CPL, OUT, AVG, T><<<pass_grid(edge_passes(CPL, L.n_edge), t), threads, 0, st>>>(
+            L, pull_offsets(L), L.rows_edge, L.n_edge, fs, fd, scale);
         return check_launch("k_edge");
     }
     return LBM_OK;
+}
+
+// The three lists in one launch (k_all_lists): whenever the call leaves the grid and the streams to
+// the launcher.  false: one launch per list.  With float32 storage and more than 96 warps per SM (six
+// waves) the special and edge passes are spread over the grid, beside the plain ones: 3.2M cells 89 us
+// a step against 92 in list order, 8M 209 against 215, but 0.2M 19 against 18.  With 16-bit storage
+// list order is the faster one at every size (3.2M cells 60 against 64, 36M 547 against 580).
+template <int CPL, bool UCOL, typename T>
+bool launch_all_lists(const lbm_lattice& L, const T* fs, T* fd, float scale, const lbm_tile& t, uint32_t mode,
+                      cudaStream_t st, int* err)
+{
+    constexpr bool F32 = std::is_same<T, float>::value;
+    if (t.ctas_per_sm > 0 || (mode & (LBM_STEP_OVERLAP | LBM_STEP_SKIP_PLAIN | LBM_STEP_SKIP_SPECIAL))) return false;
+    const long long ends = (long long)L.n_special * CPL + edge_passes(CPL, L.n_edge);
+    const long long warps = ends + (F32 ? L.n_plain : ((long long)L.n_plain * CPL + 3) / 4);
+    const long long ctas = (warps + t.warps - 1) / t.warps;
+    if (ctas == 0) return false;
+    const int nspread = F32 && warps > 96LL * sm_count() ? (int)((ends + t.warps - 1) / t.warps) : 0;
+    k_all_lists<CPL, UCOL, T><<<(unsigned)ctas, 32 * t.warps, 0, st>>>(L, pull_offsets(L), fs, fd, scale, nspread);
+    *err = check_launch("k_all_lists");
+    return true;
 }
 
 template <int V, bool OUT, bool UCOL, bool AVG>
 int launch_split_t(const lbm_lattice& L, const float* fs, float* fd, const lbm_tile& t, uint32_t mode,
                    cudaStream_t st)
 {
+    if constexpr (!OUT) {
+        int e;
+        if (launch_all_lists<V, UCOL, float>(L, fs, fd, 1.f, t, mode, st, &e)) return e;
+    }
     // LBM_STEP_OVERLAP: edge and special kernels on the side stream beside the plain kernel, whose
     // CTAs per SM tile.ctas_per_sm then limits alone
     const bool overlap = (mode & LBM_STEP_OVERLAP) && !(mode & (LBM_STEP_SKIP_PLAIN | LBM_STEP_SKIP_SPECIAL));
@@ -572,6 +597,10 @@ template <int CPL, bool OUT, bool UCOL, bool AVG>
 int launch_split_h_t(const lbm_lattice& L, const __half* hs, __half* hd, float scale, const lbm_tile& t,
                      uint32_t mode, cudaStream_t st)
 {
+    if constexpr (!OUT && CPL <= 4) {                      // wider segments and 8 cells per lane: per list
+        int e;
+        if (t.stages != 8 && launch_all_lists<CPL, UCOL, __half>(L, hs, hd, scale, t, mode, st, &e)) return e;
+    }
     // LBM_STEP_OVERLAP: edge and special kernels on the side stream beside the plain kernel, whose
     // CTAs per SM tile.ctas_per_sm then limits alone
     const bool overlap = (mode & LBM_STEP_OVERLAP) && !(mode & (LBM_STEP_SKIP_PLAIN | LBM_STEP_SKIP_SPECIAL));
@@ -668,6 +697,14 @@ template <bool OUT, bool UCOL, bool AVG>
 int launch_batch_t(const lbm_batch& b, const BatchDesc& B, int parity, uint32_t mode, const lbm_tile& t,
                    cudaStream_t st)
 {
+    const long long warps = 2LL * b.n_special + (b.n_edge + 1LL) / 2 + (b.n_plain + 1LL) / 2;
+    if (!OUT && t.stages != 8 && t.ctas_per_sm == 0 && warps > 0 &&
+        !(mode & (LBM_STEP_SKIP_PLAIN | LBM_STEP_SKIP_SPECIAL))) {
+        k_batch_all<UCOL><<<(unsigned)((warps + t.warps - 1) / t.warps), 32 * t.warps, 0, st>>>(B, parity, b);
+        if (int e = check_launch("k_batch_all")) return e;
+        k_batch_bc_rows<<<dim3((unsigned)((b.max_rows + 127) / 128), (unsigned)b.count), 128, 0, st>>>(B, parity);
+        return check_launch("k_batch_bc_rows");
+    }
     if (!(mode & LBM_STEP_SKIP_PLAIN)) {
         int e;
         if (t.stages == 8)
