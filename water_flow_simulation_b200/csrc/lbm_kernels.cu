@@ -763,8 +763,8 @@ int launch_worklists(const lbm_lattice& L, int cells_per_lane, long long n, uint
     return check_launch("k_compact");
 }
 
-// Row chunks of the profile reduction (pass 1 runs nx x chunks threads).
-int profile_chunks(const lbm_lattice& L) { return L.ny * L.nz < 256 ? L.ny * L.nz : 256; }
+// Chunks of columns of the profile reduction (pass 1 runs nx x chunks threads).
+int profile_chunks(const lbm_lattice& L) { return L.ny < 256 ? L.ny : 256; }
 
 // ---------------------------------------------------------------------------------------------
 // Static scratch of lbm_build_worklists_noalloc.
@@ -843,7 +843,7 @@ int body_forces_t(const lbm_lattice* lat, const T* f, float inv_scale, const uin
     k_body_forces<T><<<kBodyBlocks, kBodyThreads, 0, st>>>(L, f, inv_scale, nbody > 0 ? body : &no_body, nbody, ucol,
                                                            scratch);
     if (int e = check_launch("k_body_forces")) return e;
-    k_body_forces_sum<<<1, 64, 0, st>>>(scratch, kBodyBlocks, nacc, out);
+    k_body_forces_sum<<<(unsigned)nacc, 256, 0, st>>>(scratch, kBodyBlocks, out);
     return check_launch("k_body_forces_sum");
 }
 }  // namespace
@@ -1044,16 +1044,13 @@ int lbm_profiles(const lbm_lattice* lat, double inv_navg, double* prof, double* 
     if (!L.avg && (!L.rho || !L.ux || !L.uy || !L.uz)) return fail(LBM_ERR_ARG, "lbm_profiles: NULL field");
     if (!(inv_navg > 0.0)) return fail(LBM_ERR_ARG, "lbm_profiles: inv_navg must be positive");
     cudaStream_t st = as_stream(stream);
-    const int nch = profile_chunks(L);
-    const int rows = L.ny * L.nz, per = (rows + nch - 1) / nch;
-    k_profile_partials<<<dim3((unsigned)((L.nx + 127) / 128), (unsigned)nch), 128, 0, st>>>(L, inv_navg, per, scratch);
+    const int nch = profile_chunks(L), per = (L.ny + nch - 1) / nch;
+    const dim3 grid((unsigned)((L.nx + 127) / 128), (unsigned)nch);
+    if (L.avg) k_profile_partials<true><<<grid, 128, 0, st>>>(L, inv_navg, per, scratch, bed_speed2);
+    else k_profile_partials<false><<<grid, 128, 0, st>>>(L, inv_navg, per, scratch, bed_speed2);
     if (int e = check_launch("k_profile_partials")) return e;
-    const long long n = (long long)PROF_NF * L.nx;
-    k_profile_sum<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(scratch, nch, L.nx, prof);
-    if (int e = check_launch("k_profile_sum")) return e;
-    const long long m = (long long)L.nx * L.ny;
-    k_bed_speed2<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(L, inv_navg, bed_speed2);
-    return check_launch("k_bed_speed2");
+    k_profile_sum<<<(unsigned)(((long long)PROF_NF * L.nx + 31) / 32), dim3(32, 8), 0, st>>>(scratch, nch, L.nx, prof);
+    return check_launch("k_profile_sum");
 }
 
 int64_t lbm_body_forces_scratch_doubles(int nbody)

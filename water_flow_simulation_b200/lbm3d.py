@@ -361,15 +361,16 @@ class LBM3D:
         if n_scr < 0:
             nat.check(n_scr, "lbm_profiles_scratch_doubles")
         f64 = torch.float64
-        prof = torch.empty(len(nat.PROFILE_FIELDS) * self.nx, dtype=f64, device=self.device)
-        sp2 = torch.empty(self.ny * self.nx, dtype=f64, device=self.device)
+        nf = len(nat.PROFILE_FIELDS) * self.nx
+        out = torch.empty(nf + self.ny * self.nx, dtype=f64, device=self.device)     # read back in one copy
+        prof, sp2 = out[:nf], out[nf:]
         scratch = torch.empty(max(n_scr, 1), dtype=f64, device=self.device)
         inv = 1.0 / self.navg if use_avg else 1.0
         nat.check(self.lib.lbm_profiles(ref, inv, ctypes_ptr(prof), ctypes_ptr(sp2), ctypes_ptr(scratch),
                                         self._stream()), "lbm_profiles")
-        p = prof.view(len(nat.PROFILE_FIELDS), self.nx).cpu().numpy()
-        out = {k: p[i] for i, k in enumerate(nat.PROFILE_FIELDS)}
-        out["bed_speed2"] = sp2.view(self.ny, self.nx).cpu().numpy()
+        host = out.cpu().numpy()
+        out = dict(zip(nat.PROFILE_FIELDS, host[:nf].reshape(-1, self.nx)))
+        out["bed_speed2"] = host[nf:].reshape(self.ny, self.nx)
         return out
 
     def body_forces(self, body, nbody):
