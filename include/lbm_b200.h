@@ -379,7 +379,7 @@ int lbm_gemm_bf16(const uint16_t *A, int lda, const uint16_t *B, int ldb, int M,
 
 /* 3x3x3 convolutions of channels-last bf16 grids on the tensor cores, without a column matrix (tap
  * order and zero padding as below).  lbm_conv3_bf16: D[v][n] = epilogue(sum_t sum_c x[tap t of v][c]
- * W[n][t*C + c] + bias[n]), C a multiple of 64, N of 8, epilogues 2, 3 and 4 of lbm_gemm_bf16; the
+ * W[n][t*C + c] + bias[n]), C 8 or a multiple of 64, N of 8, epilogues 2, 3 and 4 of lbm_gemm_bf16; the
  * same values as that GEMM on the column matrix.  lbm_conv3_back: its gradient to the input,
  * dX[v][c] = sum_t (sum_o g[u][o] Wt[t*C + c][o]) over the (u, t) that read v, Wt the transposed
  * weights (27*C x O), O a multiple of 8, C of 64.  Pointers 16-byte aligned; err as lbm_gemm_bf16's. */

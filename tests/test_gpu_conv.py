@@ -81,3 +81,10 @@ def test_argument_errors():
     assert lib.lbm_conv3_bf16(p + 2, 64, 2, 1, 1, p, 8, p, 2, b, e, st) == -1        # alignment
     assert lib.lbm_conv3_back(p, 8, 2, 1, 1, p, 72, p, e, st) == -1
     assert lib.lbm_nn_im2col_t(p, 8, 2, 1, 1, 12, p, st) == -1
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("cout", (8, 40, 64, 72))
+@pytest.mark.parametrize("epi", (2, 3, 4))
+def test_input_layer_equals_the_column_matrix_product(cout, grid, epi):
+    test_forward_equals_the_column_matrix_product(8, cout, grid, epi)

@@ -137,13 +137,8 @@ class SurrogateNet:
         P = self.p[name]
         y = torch.empty(V, cout, dtype=torch.float32 if f32_out else torch.bfloat16, device=self.device)
         epi = 4 if f32_out else 3 if relu else 2
-        if cin % 64 == 0:
-            nat.check(self.lib.lbm_conv3_bf16(x.data_ptr(), cin, X, Y, Z, P["Wb"].data_ptr(), cout, y.data_ptr(), epi,
-                                              P["b"].data_ptr(), self.err.data_ptr(), self._st()), "lbm_conv3_bf16")
-        else:                               # the input layer's 8 channels: through a column matrix
-            col = torch.empty(V, 27 * cin, dtype=torch.bfloat16, device=self.device)
-            nat.check(self.lib.lbm_nn_im2col(x.data_ptr(), cin, X, Y, Z, col.data_ptr(), self._st()), "lbm_nn_im2col")
-            self._gemm(col, 27 * cin, P["Wb"], 27 * cin, V, cout, 27 * cin, y, cout, epi, P["b"])
+        nat.check(self.lib.lbm_conv3_bf16(x.data_ptr(), cin, X, Y, Z, P["Wb"].data_ptr(), cout, y.data_ptr(), epi,
+                                          P["b"].data_ptr(), self.err.data_ptr(), self._st()), "lbm_conv3_bf16")
         self.cache[name] = (x, y, dims, cin, cout, relu)
         return y
 
