@@ -88,3 +88,36 @@ def test_argument_errors():
 @pytest.mark.parametrize("epi", (2, 3, 4))
 def test_input_layer_equals_the_column_matrix_product(cout, grid, epi):
     test_forward_equals_the_column_matrix_product(8, cout, grid, epi)
+
+
+@pytest.mark.parametrize("C", (8, 12, 64))
+@pytest.mark.parametrize("grid", ((2, 2, 2), (2, 6, 10), (4, 8, 66)))
+def test_pooling_and_upsampling(C, grid):
+    """Sums of eight in index order in float32, one rounding to bf16: equal to the same sums in torch."""
+    torch, nat, lib, _, st = setup(8, 8, (1, 1, 1))
+    Z, Y, X = grid
+    g = torch.Generator(device="cuda").manual_seed(C + X)
+    full = torch.randn(Z, Y, X, C, device="cuda", generator=g).to(torch.bfloat16)
+    half = torch.randn(Z // 2, Y // 2, X // 2, C, device="cuda", generator=g).to(torch.bfloat16)
+
+    def children(a):
+        s = torch.zeros_like(half, dtype=torch.float32)
+        for d in range(8):
+            s = s + a[d >> 2::2, d >> 1 & 1::2, d & 1::2].float()
+        return s
+
+    def up(a):
+        return a[:, None, :, None, :, None].expand(-1, 2, -1, 2, -1, 2, -1).reshape(Z, Y, X, C)
+    out_h, out_f = torch.empty_like(half), torch.empty_like(full)
+    nat.check(lib.lbm_nn_pool2(full.data_ptr(), C, X, Y, Z, out_h.data_ptr(), st), "pool2")
+    assert torch.equal(out_h, (0.125 * children(full)).to(torch.bfloat16))
+    nat.check(lib.lbm_nn_up2_add(half.data_ptr(), full.data_ptr(), C, X, Y, Z, out_f.data_ptr(), st), "up2_add")
+    assert torch.equal(out_f, (up(half).float() + full.float()).to(torch.bfloat16))
+    ff, hf = full.float(), half.float()
+    out_hf = torch.empty_like(hf)
+    nat.check(lib.lbm_nn_up2_back(ff.data_ptr(), C, X, Y, Z, out_hf.data_ptr(), st), "up2_back")
+    assert torch.equal(out_hf, children(ff))
+    for acc in (0, 1):
+        out_ff = ff.clone()
+        nat.check(lib.lbm_nn_pool2_back(hf.data_ptr(), C, X, Y, Z, out_ff.data_ptr(), acc, st), "pool2_back")
+        assert torch.equal(out_ff, 0.125 * up(hf) + (ff if acc else 0))
