@@ -754,7 +754,8 @@ int launch_worklists(const lbm_lattice& L, int cells_per_lane, long long n, uint
                      uint32_t* solid, uint32_t* special, uint32_t* edge, int32_t* counts, cudaStream_t st)
 {
     const int per_block = cells_per_lane == 2 ? 16 : 8;         // segments of 256 threads
-    k_classify<<<(unsigned)((n + per_block - 1) / per_block), 256, 0, st>>>(L, cells_per_lane, scratch);
+    const int per_grid_step = per_block * kClassAhead;
+    k_classify<<<(unsigned)((n + per_grid_step - 1) / per_grid_step), 256, 0, st>>>(L, cells_per_lane, scratch);
     if (int e = check_launch("k_classify")) return e;
     // chunks of at least 2048 entries, a multiple of 16 each, over at most one CTA per SM
     long long chunk = (n + sm_count() - 1) / sm_count();
@@ -911,10 +912,10 @@ int lbm_pitch_rows(const void* src, void* dst, int elem_bytes, int nx, int pitch
     if (((reinterpret_cast<uintptr_t>(dst) | (elem_bytes == 4 ? reinterpret_cast<uintptr_t>(src) : 0)) & 3) != 0)
         return fail(LBM_ERR_ARG, "lbm_pitch_rows: arrays must be 4-byte aligned");
     if (elem_bytes == 4)
-        k_pitch_rows<uint32_t><<<row_grid(rows, pitch), 128, 0, as_stream(stream)>>>(
+        k_pitch_rows<uint32_t><<<row_grid((rows + kPitchRows - 1) / kPitchRows, pitch), 128, 0, as_stream(stream)>>>(
             static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), nx, pitch, rows, pad);
     else
-        k_pitch_rows<uint8_t><<<row_grid(rows, pitch), 128, 0, as_stream(stream)>>>(
+        k_pitch_rows<uint8_t><<<row_grid((rows + kPitchRows - 1) / kPitchRows, pitch), 128, 0, as_stream(stream)>>>(
             static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), nx, pitch, rows, (uint8_t)pad);
     return check_launch("lbm_pitch_rows");
 }

@@ -20,19 +20,28 @@ dim3 row_grid(long long rows, int pitch)
     return dim3((unsigned)((pitch / 4 + 127) / 128), gy, (unsigned)((rows + gy - 1) / gy));
 }
 
-// Rows of nx elements (1 or 4 bytes each) to rows of `pitch`, the rest filled with `pad`.
+// Rows of nx elements (1 or 4 bytes each) to rows of `pitch`, the rest filled with `pad`.  A thread takes
+// four cells of kPitchRows consecutive rows, all requested together: with one row a thread the
+// blocks came and went 30 deep, each waiting for one load (36M cells: bytes 40 -> 25 us, floats 58 -> 46).
+constexpr int kPitchRows = 4;
+
 template <typename T>
 __global__ void __launch_bounds__(128) k_pitch_rows(const T* __restrict__ src, T* __restrict__ dst, int nx, int pitch,
                                                     long long rows, T pad)
 {
-    long long row;
+    long long group;
     int x;
-    if (!row_of(rows, pitch, row, x)) return;
-    const T* s = src + row * nx + x;
-    struct __align__(4) Four { T v[4]; } o;
+    if (!row_of((rows + kPitchRows - 1) / kPitchRows, pitch, group, x)) return;
+    const long long row0 = group * kPitchRows;
+    struct __align__(4) Four { T v[4]; } o[kPitchRows];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) o.v[k] = x + k < nx ? __ldg(s + k) : pad;
-    *reinterpret_cast<Four*>(dst + row * pitch + x) = o;
+    for (int j = 0; j < kPitchRows; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            o[j].v[k] = row0 + j < rows && x + k < nx ? __ldg(src + (row0 + j) * nx + x + k) : pad;
+#pragma unroll
+    for (int j = 0; j < kPitchRows; ++j)
+        if (row0 + j < rows) *reinterpret_cast<Four*>(dst + (row0 + j) * pitch + x) = o[j];
 }
 
 // Cell flags from unvectorised accesses: arrays at any alignment.
@@ -135,49 +144,66 @@ __global__ void __launch_bounds__(128) k_build_flags4(const lbm_lattice L, const
     *reinterpret_cast<uint4*>(flags + c) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
-// 0 plain, 1 solid, 2 special, 3 edge (see fused_split.cuh): 8*V lanes (at most 32) of four flags
-// each per segment of 32*V cells; one flag at a time where they are not 16-byte aligned.
+// Four flags: one access, or one flag at a time where they are not 16-byte aligned.
+__device__ __forceinline__ void load_flags4(uint32_t (&fk)[4], const uint32_t* p, bool vec)
+{
+    if (vec) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+        fk[0] = v.x; fk[1] = v.y; fk[2] = v.z; fk[3] = v.w;
+    } else {
+        for (int k = 0; k < 4; ++k) fk[k] = __ldg(p + k);
+    }
+}
+
+// 0 plain, 1 solid, 2 special, 3 edge (see fused_split.cuh): 8*V lanes (at most 32) of four flags each
+// per segment of 32*V cells, kClassAhead segments in flight per thread (36M cells: 75 us, 99
+// with one).
+constexpr int kClassAhead = 4;
 __global__ void __launch_bounds__(256) k_classify(const lbm_lattice L, int V, uint8_t* __restrict__ cls)
 {
     const int SEG = 32 * V, G = V >= 4 ? 32 : 8 * V, lane = threadIdx.x & 31, gl = lane % G;
     const int nseg = (L.pitch + SEG - 1) / SEG;
     const long long n = (long long)nseg * L.ny * L.nz;
-    const long long id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    const bool valid = id < n;
-    const uint32_t id32 = valid ? (uint32_t)id : 0u;       // ids are 32-bit
-    const int seg = (int)(id32 % (uint32_t)nseg);
-    const uint32_t yz = id32 / (uint32_t)nseg;
-    const int y = (int)(yz % (uint32_t)L.ny), z = (int)(yz / (uint32_t)L.ny);
-    const long long rowc = (long long)yz * L.pitch;
-    const int xa = seg * SEG, xb = min(xa + SEG, L.pitch);
+    const long long id0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / G, step = (long long)gridDim.x * blockDim.x / G;
     const bool vec = (reinterpret_cast<uintptr_t>(L.flags) & 15) == 0;
-    bool fluid_seen = false, any_special = false;
-    for (int x = xa + 4 * gl; x < xb; x += 4 * G) {
-        uint32_t fk[4];
-        if (vec) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(L.flags + rowc + x));
-            fk[0] = v.x; fk[1] = v.y; fk[2] = v.z; fk[3] = v.w;
-        } else {
-            for (int k = 0; k < 4; ++k) fk[k] = __ldg(L.flags + rowc + x + k);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            fluid_seen |= (fk[k] & FLAG_SOLID) == 0;
-            if (x + k < L.nx) any_special |= (fk[k] & (FLAG_SOLID | FLAG_WALLS | FLAG_WALLFN | FLAG_FORCE)) != 0;
-        }
-    }
     const unsigned group = (G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (lane - gl));
-    const bool all_solid = (__ballot_sync(0xffffffffu, fluid_seen) & group) == 0;
-    any_special = (__ballot_sync(0xffffffffu, any_special) & group) != 0;
-    // open rows: clear of the y walls and the bed; the row under the lid counts (its -z movers
-    // read the own row's mirrored populations at constant offsets)
-    if (L.sponge_cols > 0 && xb > L.nx - L.sponge_cols) any_special = true;   // per-cell relaxation time
-    const bool interior_row = y >= 1 && y <= L.ny - 2 && z >= 1 && z <= L.nz - 1;
-    const bool clear_of_edges = seg > 0 && xa + SEG < L.nx;
-    int c = 2;
-    if (all_solid) c = 1;
-    else if (interior_row && !any_special) c = clear_of_edges ? 0 : 3;
-    if (valid && gl == 0) cls[id] = (uint8_t)c;
+    uint32_t fk[kClassAhead][4];                           // the first four flags of each segment, requested together
+#pragma unroll
+    for (int j = 0; j < kClassAhead; ++j) {
+        const uint32_t id = id0 + j * step < n ? (uint32_t)(id0 + j * step) : 0u;            // ids are 32-bit
+        const int x = (int)(id % (uint32_t)nseg) * SEG + 4 * gl;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) fk[j][k] = FLAG_GHOST | FLAG_SOLID;
+        if (x < L.pitch) load_flags4(fk[j], L.flags + (long long)(id / (uint32_t)nseg) * L.pitch + x, vec);
+    }
+#pragma unroll
+    for (int j = 0; j < kClassAhead; ++j) {
+        const long long id = id0 + j * step;
+        const bool valid = id < n;
+        const uint32_t id32 = valid ? (uint32_t)id : 0u, yz = id32 / (uint32_t)nseg;
+        const int seg = (int)(id32 % (uint32_t)nseg), y = (int)(yz % (uint32_t)L.ny), z = (int)(yz / (uint32_t)L.ny);
+        const int xa = seg * SEG, xb = min(xa + SEG, L.pitch);
+        bool fluid_seen = false, any_special = false;
+        for (int x = xa + 4 * gl; x < xb; x += 4 * G) {
+            if (x != xa + 4 * gl) load_flags4(fk[j], L.flags + (long long)yz * L.pitch + x, vec);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                fluid_seen |= (fk[j][k] & FLAG_SOLID) == 0;
+                if (x + k < L.nx) any_special |= (fk[j][k] & (FLAG_SOLID | FLAG_WALLS | FLAG_WALLFN | FLAG_FORCE)) != 0;
+            }
+        }
+        const bool all_solid = (__ballot_sync(0xffffffffu, fluid_seen) & group) == 0;
+        any_special = (__ballot_sync(0xffffffffu, any_special) & group) != 0;
+        // open rows: clear of the y walls and the bed; the row under the lid counts (its -z movers
+        // read the own row's mirrored populations at constant offsets)
+        if (L.sponge_cols > 0 && xb > L.nx - L.sponge_cols) any_special = true;   // per-cell relaxation time
+        const bool interior_row = y >= 1 && y <= L.ny - 2 && z >= 1 && z <= L.nz - 1;
+        const bool clear_of_edges = seg > 0 && xa + SEG < L.nx;
+        int c = 2;
+        if (all_solid) c = 1;
+        else if (interior_row && !any_special) c = clear_of_edges ? 0 : 3;
+        if (valid && gl == 0) cls[id] = (uint8_t)c;
+    }
 }
 
 // Ordered stream compaction of the four classes.  CTA b takes `chunk` entries (a multiple of 16)
