@@ -40,3 +40,28 @@ def test_one_launch_equals_a_launch_per_list(storage, cells, warps, dims, column
         L.step(4, accumulate=True)
         got.append([t.clone().view(torch.uint8) for t in (L.f, L.f2, L.rho, L.ux, L.uy, L.uz, L.avg_sum("sp"))])
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("dims", ((16, 5, 4), (300, 40, 9), (620, 150, 24)))
+@pytest.mark.parametrize("storage", ("fp32", "fp16"))
+def test_steps_back_to_back_equal_steps_one_by_one(storage, dims):
+    """Steps launched while the one before drains (lattices of up to 5M cells), against the same steps each
+    waited for: every step reads the whole of the last one's populations and wall fields."""
+    from water_flow_simulation_b200 import _native as nat
+    got = []
+    for wait in (False, True):
+        torch, L = lattice(dims, (nat.PIPE_SPLIT, 2, 4, 0, 0) if storage == "fp16" else None, True, storage)
+        if wait:
+            tile, st = L.tile, L._stream()
+            lat = L._lattice_ref()
+            step = L.lib.lbm_fused_step_h if storage == "fp16" else L.lib.lbm_fused_step
+            scale = (L.store_scale,) if storage == "fp16" else ()
+            for _ in range(120):
+                nat.check(step(lat, L.f.data_ptr(), L.f2.data_ptr(), *scale, nat.STEP_UREF_COLUMN, tile, st), "step")
+                torch.cuda.synchronize()
+                L.f, L.f2 = L.f2, L.f
+            L.step(1)
+        else:
+            L.step(121)
+        got.append([t.clone().view(torch.uint8) for t in (L.f, L.f2, L.rho, L.ux, L.uy, L.uz)])
+    assert all(torch.equal(a, b) for a, b in zip(*got))

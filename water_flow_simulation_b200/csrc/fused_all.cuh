@@ -23,7 +23,7 @@
 // the edge list's, then the plain list's; the code of each pass is that of k_cells, k_edge, k_rows
 // and k_rows_h_plain, and the lists' passes do not read what another writes.  `nspread` > 0: the
 // first nspread CTAs' worth of passes (special and edge) are spread evenly over the grid.
-template <int CPL, bool UCOL, typename T>
+template <int CPL, bool UCOL, bool EARLY, typename T>
 __global__ void __launch_bounds__(128, std::is_same<T, float>::value ? 4 : 5)
     k_all_lists(const lbm_lattice L, const PullOffsets po, const T* __restrict__ fs, T* __restrict__ fd, float scale,
                 int nspread)
@@ -32,6 +32,12 @@ __global__ void __launch_bounds__(128, std::is_same<T, float>::value ? 4 : 5)
     constexpr bool F32 = std::is_same<T, float>::value;
     const int lane = threadIdx.x & 31, nseg = (L.pitch + SEG - 1) / SEG;
     const float inv_scale = 1.0f / scale;
+    if constexpr (EARLY) {
+        // launched while the step before is in its last wave (launch_all_lists): nothing is read or written
+        // until that step has ended, and the next one may start once every CTA of this one has
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     int cta = (int)blockIdx.x;
     if (nspread > 0) {
         const int before = (int)((long long)cta * nspread / gridDim.x);

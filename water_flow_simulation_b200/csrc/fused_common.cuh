@@ -82,7 +82,7 @@ __device__ __forceinline__ void vload_plain(float (&o)[V], const float* p)
 // ---------------------------------------------------------------------------------------------
 template <int V>
 __device__ __forceinline__ void ldv(float (&o)[V], const float* p) { Vec<V>::load(o, p); }
-__device__ __forceinline__ float ld1(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float ld1(const float* p) { return __ldca(p); }
 
 __device__ __forceinline__ float2 half2_bits_to_float2(uint32_t b)
 {
@@ -98,7 +98,7 @@ __device__ __forceinline__ uint32_t float2_to_half2_bits(float lo, float hi)
     return b;
 }
 
-__device__ __forceinline__ float ld1(const __half* p) { return __half2float(__ldg(p)); }
+__device__ __forceinline__ float ld1(const __half* p) { return __half2float(__ldca(p)); }
 
 // 16-bit storage read through coherent loads (ld.global.cg, served by L2): for a kernel that
 // reads populations which other CTAs wrote earlier in the same launch (the persistent batch
@@ -136,47 +136,48 @@ __device__ __forceinline__ long long pull_offset(const PullOffsets& po, bool lid
     else return po.d[I];
 }
 
-// Read-only loads that keep their order: the plain kernels issue all of a segment's loads before
+// Population loads that keep their order (coherent ones: k_all_lists may start before the step that
+// wrote them has ended, and waits for it): the plain kernels issue all of a segment's loads before
 // the first shuffle or conversion waits for one.  The predicated ones leave `v` as it is in the
 // lanes where `on` is false.
 __device__ __forceinline__ void ld_ordered(uint32_t (&v)[1], const void* p)
 {
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v[0]) : "l"(p));
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v[0]) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered(uint32_t (&v)[2], const void* p)
 {
-    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered(uint32_t (&v)[4], const void* p)
 {
-    asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered_if(bool on, uint32_t& v, const void* p)
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.u32 %0, [%1];\n\t}"
                  : "+r"(v) : "l"(p), "r"((uint32_t)on));
 }
 __device__ __forceinline__ void ld_ordered(uint16_t& v, const void* p)
 {
-    asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered(float& v, const void* p)
 {
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered(float (&v)[2], const void* p)
 {
-    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered(float (&v)[4], const void* p)
 {
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
 __device__ __forceinline__ void ld_ordered_if(bool on, float& v, const void* p)
 {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}"
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.global.f32 %0, [%1];\n\t}"
                  : "+f"(v) : "l"(p), "r"((uint32_t)on));
 }
 
