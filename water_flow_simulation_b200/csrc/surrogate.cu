@@ -764,7 +764,8 @@ int launch_gemm_any(int bn, const __nv_bfloat16* A, int lda, const __nv_bfloat16
 // k_im2col do, so the accumulation and the results are those of the GEMM on the column matrix.
 // What bounds it: the 27 shifted reads of the grid now come from L2 instead of the column matrix's
 // write and read in HBM (415 MB each way for 64 channels on 120k voxels).  A prediction on 120k
-// voxels (10 x 80 x 150) takes 389 us instead of 1069, a gradient on 12k voxels 816 instead of 1099.
+// voxels (10 x 80 x 150) took 389 us instead of 1069, a gradient on 12k voxels 816 instead of 1099; with the
+// input layer, pooling and issue below 216 and 800 (whose loss adds 56 us of atomics).
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
                                             uint32_t mbar)
