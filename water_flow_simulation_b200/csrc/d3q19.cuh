@@ -36,6 +36,24 @@ __host__ __device__ constexpr double wgt64(int i) {
     return i == 0 ? 1.0 / 3.0 : (i < 7 ? 1.0 / 18.0 : 1.0 / 36.0);
 }
 
+// Element of the population array (19 planes of S cells) that direction I pulls for the cell with
+// element index `own` in a plane (fk its flag word): at a wall the opposite population of the cell
+// itself, across an x end the cell's own, under the lid the mirrored one, else the neighbour's.
+// The planes' bases and the offsets are uniform, so a lane selects one and adds.  64-bit sums: the
+// opposite direction's plane is S cells away, so own and offset together pass 2^31 on lattices of
+// more than 2^30 cells (16-bit storage of 1.5e9 cells fits one GPU).
+template <int I>
+__host__ __device__ __forceinline__ long long pull_element(long long own, long long plane, int pitch, long long S,
+                                                           uint32_t fk, bool lid, bool x_first, bool x_last)
+{
+    const bool edge = cx(I) == 1 ? x_first : cx(I) == -1 ? x_last : false;
+    long long off = I * S - (cz(I) * plane + (long long)cy(I) * pitch + cx(I));
+    if (cz(I) == -1) off = lid ? mirz(I) * S - ((long long)cy(I) * pitch + cx(I)) : off;
+    if (cx(I)) off = edge ? I * S : off;
+    if (I > 0) off = (fk & (1u << I)) ? opp(I) * S : off;
+    return own + off;
+}
+
 // Cell flag word (one uint32 per cell).
 constexpr uint32_t FLAG_WALLS = 0x0007FFFEu;   // bit i (1..18): pull source of direction i is a wall
 constexpr uint32_t FLAG_SOLID = 1u << 19;      // solid cell (never collided)

@@ -14,11 +14,6 @@
 // four cells per lane with a branch, and a dependent load, per bounced direction.
 #pragma once
 
-// Population of direction I pulled for the cell with element index `own` in a direction's plane
-// (fk its flag word): at a wall the opposite one of the cell itself, across an x end the cell's
-// own, under the lid the mirrored one, else the neighbour's.  The planes' bases are uniform and
-// the opposite direction's plane is the next or the last one, so the address of a lane is one
-// 32-bit select, an add and a widening multiply-add (cells < 2^31 on any GPU of 180 GB).
 // One stored population as it lies in memory, and its value as float.
 template <typename T> struct Stored {
     using type = uint16_t;
@@ -35,30 +30,13 @@ __device__ __forceinline__ void load_cell(uint16_t& v, const hcoh* p)
     v = __half_as_ushort(__ldcg(reinterpret_cast<const __half*>(p)));
 }
 
-template <int I, typename T>
-__device__ __forceinline__ const T* pull_cell(const T* __restrict__ fs, int own, int plane, int pitch, long long S,
-                                              uint32_t fk, bool lid, bool x_first, bool x_last)
-{
-    const bool wall = I > 0 && (fk & (1u << I));
-    const bool edge = cx(I) == 1 ? x_first : cx(I) == -1 ? x_last : false;
-    if constexpr (cz(I) == -1) {                           // the lid's mirrored plane may be two away
-        long long off = lid ? (mirz(I) - I) * S - (cy(I) * pitch + cx(I)) : plane - (cy(I) * pitch + cx(I));
-        if (cx(I)) off = edge ? 0 : off;
-        off = wall ? (opp(I) - I) * S : off;
-        return fs + I * S + own + off;
-    }
-    int off = -(cz(I) * plane + cy(I) * pitch + cx(I));
-    if (cx(I)) off = edge ? 0 : off;
-    if (I > 0) off = wall ? (opp(I) - I) * (int)S : off;
-    return fs + I * S + (own + off);
-}
 template <typename T, int... Is>
 __device__ __forceinline__ void pull_cell_all(std::integer_sequence<int, Is...>, float (&f)[Q],
-                                              const T* __restrict__ fs, int own, int plane, int pitch, long long S,
-                                              uint32_t fk, bool lid, bool x_first, bool x_last)
+                                              const T* __restrict__ fs, long long own, long long plane, int pitch,
+                                              long long S, uint32_t fk, bool lid, bool x_first, bool x_last)
 {
     typename Stored<T>::type v[Q];
-    (load_cell(v[Is], pull_cell<Is, T>(fs, own, plane, pitch, S, fk, lid, x_first, x_last)), ...);
+    (load_cell(v[Is], fs + pull_element<Is>(own, plane, pitch, S, fk, lid, x_first, x_last)), ...);
     ((f[Is] = Stored<T>::value(v[Is])), ...);
 }
 
@@ -76,7 +54,7 @@ __device__ __forceinline__ void store_cell(hcoh* p, float v, float scale)
     store_cell<I>(reinterpret_cast<__half*>(p), v, scale);
 }
 template <typename T, int... Is>
-__device__ __forceinline__ void store_cell_all(std::integer_sequence<int, Is...>, T* fd, int own, long long S,
+__device__ __forceinline__ void store_cell_all(std::integer_sequence<int, Is...>, T* fd, long long own, long long S,
                                                const float (&f)[Q], float scale)
 {
     (store_cell<Is>(fd + Is * S + own, f[Is], scale), ...);
@@ -103,7 +81,7 @@ __device__ __forceinline__ void cell_pass(const lbm_lattice& L, const T* __restr
     const long long S = L.cells;
     const int x = xa + lane;
     const bool active = x < L.pitch, solid = (fk & FLAG_SOLID) != 0;
-    const int plane = L.ny * L.pitch, own = z * plane + y * L.pitch + x;
+    const long long plane = (long long)L.ny * L.pitch, own = z * plane + (long long)y * L.pitch + x;
     float f[Q];
     float r = 1.f, ux = 0.f, uy = 0.f, uz = 0.f;
     if (!solid) {
