@@ -25,6 +25,7 @@
 #include <cstdint>
 
 #include "errors.cuh"
+#include "shared_mem.cuh"
 #include "../../include/lbm_b200.h"
 
 using namespace wfs;
@@ -397,11 +398,8 @@ int launch_gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb
 {
     auto kern = k_gemm_bf16<BN, EPI>;
     const int smem = GM * 128 + BN * 128 + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr_set = true;
-    }
+    if (const cudaError_t e = allow_shared(kern, smem))
+        return fail(LBM_ERR_CUDA, "k_gemm_bf16: %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
     dim3 grid((unsigned)((M + GM - 1) / GM), (unsigned)((N + BN - 1) / BN));
     kern<<<grid, 128, smem, st>>>(A, lda, B, ldb, M, N, K, D, ldd, bias, err);
     return check_launch("k_gemm_bf16");
@@ -451,11 +449,7 @@ bool launch_gemm_tma(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, in
     if (!bf16_tile_map(&ta, A, M, K, lda, GM) || !bf16_tile_map(&tb, B, N, K, ldb, BN)) return false;
     auto kern = k_gemm_tma<BN, EPI, S>;
     const int smem = S * (GM * 128 + BN * 128) + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
-        attr_set = true;
-    }
+    if (allow_shared(kern, smem) != cudaSuccess) return false;
     dim3 grid((unsigned)((M + GM - 1) / GM), (unsigned)((N + BN - 1) / BN));
     kern<<<grid, 128, smem, st>>>(ta, tb, M, N, K, D, ldd, bias, err);
     *status = check_launch("k_gemm_tma");
@@ -726,10 +720,7 @@ bool launch_gemm_ws(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int
     CUtensorMap ta, tb;
     if (!bf16_tile_map(&ta, A, M, K, lda, bv) || !bf16_tile_map(&tb, B, N, K, ldb, GM)) return false;
     auto kern = k_gemm_ws<EPI>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    if (allow_shared(kern, smem) != cudaSuccess) return false;
     const long long tiles = (long long)((M + bv - 1) / bv) * ((N + GM - 1) / GM);
     const int grid = (int)(tiles < nsm ? tiles : nsm);
     kern<<<grid, kWsThreads, smem, st>>>(ta, tb, M, N, K, bv, stages, D, ldd, bias, err);
@@ -1214,8 +1205,8 @@ int launch_conv_bn(const __nv_bfloat16* x, int C, const ConvTiles& g, const __nv
         return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: no tensor map for this grid");
     auto kern = k_conv_fwd<BN, EPI, S>;
     const int smem = S * (GM * 128 + BN * 128) + 1024;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: %d bytes of shared memory: %s", smem, cudaGetErrorString(cudaGetLastError()));
+    if (const cudaError_t e = allow_shared(kern, smem))
+        return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
     kern<<<dim3((unsigned)(g.nx * g.ny * g.nz), (unsigned)((N + BN - 1) / BN)), 128, smem, st>>>(tx, tw, g, C, N, D, bias, err);
     return check_launch("k_conv_fwd");
 }
@@ -1228,8 +1219,8 @@ int launch_conv_in(const __nv_bfloat16* x, int X, int Y, int Z, const __nv_bfloa
     if (!bf16_tile_map(&tw, W, N, 27 * 8, 27 * 8, BN)) return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: no tensor map for the weights");
     auto kern = k_conv_in<BN, EPI>;
     const int smem = kInTiles * (GM * 128 + BN * 128) + 1024;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: %d bytes of shared memory: %s", smem, cudaGetErrorString(cudaGetLastError()));
+    if (const cudaError_t e = allow_shared(kern, smem))
+        return fail(LBM_ERR_CUDA, "lbm_conv3_bf16: %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
     const long long V = (long long)X * Y * Z;
     kern<<<dim3((unsigned)((V + GM - 1) / GM), (unsigned)((N + BN - 1) / BN)), 128, smem, st>>>(x, tw, X, Y, Z, N, D, bias, err);
     return check_launch("k_conv_in");
@@ -1647,8 +1638,8 @@ int lbm_conv3_back(const uint16_t* g, int O, int X, int Y, int Z, const uint16_t
         !bf16_tile_map(&tw, reinterpret_cast<const __nv_bfloat16*>(Wt), 27 * C, O, O, kBackN))
         return fail(LBM_ERR_CUDA, "lbm_conv3_back: no tensor map for this grid");
     const int smem = kBackStages * (GM * 128 + kBackN * 128) + 1024;
-    if (cudaFuncSetAttribute(k_conv_back, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-        return fail(LBM_ERR_CUDA, "lbm_conv3_back: %d bytes of shared memory: %s", smem, cudaGetErrorString(cudaGetLastError()));
+    if (const cudaError_t e = allow_shared(k_conv_back, smem))
+        return fail(LBM_ERR_CUDA, "lbm_conv3_back: %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
     k_conv_back<<<dim3((unsigned)(t.nx * t.ny * t.nz), (unsigned)(C / kBackN)), kWsThreads, smem,
                   reinterpret_cast<cudaStream_t>(stream)>>>(tg, tw, t, O, C, dX, err);
     return check_launch("k_conv_back");
