@@ -26,6 +26,7 @@
 
 #include "errors.cuh"
 #include "shared_mem.cuh"
+#include "tensor_map.cuh"
 #include "../../include/lbm_b200.h"
 
 using namespace wfs;
@@ -403,24 +404,6 @@ int launch_gemm(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb
     dim3 grid((unsigned)((M + GM - 1) / GM), (unsigned)((N + BN - 1) / BN));
     kern<<<grid, 128, smem, st>>>(A, lda, B, ldb, M, N, K, D, ldd, bias, err);
     return check_launch("k_gemm_bf16");
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (the library links no libcuda).
-using PfnEncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-PfnEncodeTiled encode_tiled()
-{
-    static PfnEncodeTiled fn = nullptr;
-    static bool resolved = false;
-    if (!resolved) {
-        resolved = true;
-        void* p = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, nullptr) ==
-            cudaSuccess)
-            fn = reinterpret_cast<PfnEncodeTiled>(p);
-    }
-    return fn;
 }
 
 // Tensor map of a rows x K bf16 matrix with row stride ld (elements), boxes of 64 (K) x box_rows,
