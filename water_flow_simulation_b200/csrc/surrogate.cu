@@ -24,6 +24,7 @@
 
 #include <cstdint>
 
+#include "channels.cuh"
 #include "errors.cuh"
 #include "shared_mem.cuh"
 #include "tensor_map.cuh"
@@ -801,16 +802,8 @@ __device__ __forceinline__ void conv_store(uint32_t lane_addr, long long v, int 
                 if constexpr (EPI == EPI_BF16_BIAS_RELU) o[j] = fmaxf(o[j], 0.f);
             }
             const size_t at = (size_t)v * N + n0 + c0 + q;
-            if constexpr (EPI == EPI_F32_BIAS) {
-                float4* d = reinterpret_cast<float4*>(static_cast<float*>(D) + at);
-                d[0] = make_float4(o[0], o[1], o[2], o[3]);
-                d[1] = make_float4(o[4], o[5], o[6], o[7]);
-            } else {
-                __nv_bfloat16 h[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16_rn(o[j]);
-                *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(D) + at) = *reinterpret_cast<uint4*>(h);
-            }
+            if constexpr (EPI == EPI_F32_BIAS) store_n<8>(static_cast<float*>(D) + at, o);
+            else store_n<8>(static_cast<__nv_bfloat16*>(D) + at, o);
         }
     }
 }
@@ -1358,56 +1351,6 @@ __global__ void k_act_grad_wide(const float* __restrict__ dY, const __nv_bfloat1
     if (relu && !(__bfloat162float(Y[i]) > 0.f)) v = 0.f;
     g[i] = __float2bfloat16_rn(v);
     atomicAdd(dbias + (i % C), v);
-}
-
-// N channels of a voxel as floats and back: one 16- or 2 x 16-byte access for N = 8 (aligned rows of a
-// multiple of 8 channels), one element for N = 1.
-template <int N>
-__device__ __forceinline__ void load_n(float (&v)[N], const __nv_bfloat16* p)
-{
-    if constexpr (N == 8) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
-        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            v[2 * j] = __uint_as_float(w[j] << 16);
-            v[2 * j + 1] = __uint_as_float(w[j] & 0xffff0000u);
-        }
-    } else {
-        v[0] = __bfloat162float(*p);
-    }
-}
-template <int N>
-__device__ __forceinline__ void load_n(float (&v)[N], const float* p)
-{
-    if constexpr (N == 8) {
-        *reinterpret_cast<float4*>(v) = reinterpret_cast<const float4*>(p)[0];
-        *reinterpret_cast<float4*>(v + 4) = reinterpret_cast<const float4*>(p)[1];
-    } else {
-        v[0] = *p;
-    }
-}
-template <int N>
-__device__ __forceinline__ void store_n(__nv_bfloat16* p, const float (&v)[N])
-{
-    if constexpr (N == 8) {
-        __align__(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16_rn(v[j]);
-        *reinterpret_cast<uint4*>(p) = *reinterpret_cast<uint4*>(h);
-    } else {
-        *p = __float2bfloat16_rn(v[0]);
-    }
-}
-template <int N>
-__device__ __forceinline__ void store_n(float* p, const float (&v)[N])
-{
-    if constexpr (N == 8) {
-        reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-    } else {
-        *p = v[0];
-    }
 }
 
 // Pooling and upsampling are copies with a few additions, bound by their bytes: a thread takes N = 8
