@@ -382,7 +382,7 @@ int launch_tma_t(const lbm_lattice& L, const float* fs, float* fd, const lbm_til
     auto kern = k_fused_tma<C, OUT, UCOL, AVG>;
     const int threads = 32 * (C + 1);
     const TmaLayout lay(32 * C, t.stages);
-    if (allow_shared(kern, lay.bytes) != cudaSuccess)
+    if (raise_shared(kern, lay.bytes) != cudaSuccess)
         return fail(LBM_ERR_ARG, "k_fused_tma: %zu bytes of shared memory not available", lay.bytes);
     const int per_sm = occupancy(kern, threads, lay.bytes, t.ctas_per_sm);
     const long long nseg = (L.pitch + 32 * C - 1) / (32 * C);
@@ -425,7 +425,7 @@ int launch_async_t(const lbm_lattice& L, const float* fs, float* fd, const lbm_t
     auto kern = k_fused_async<OUT, UCOL, AVG, D>;
     const int threads = 32 * t.warps;
     const AsyncLayout lay(t.warps, D);
-    if (allow_shared(kern, lay.bytes) != cudaSuccess)
+    if (raise_shared(kern, lay.bytes) != cudaSuccess)
         return fail(LBM_ERR_ARG, "k_fused_async: %zu bytes of shared memory not available", lay.bytes);
     const PullOffsets po = pull_offsets(L);
     const int per_sm = occupancy(kern, threads, lay.bytes, t.ctas_per_sm);

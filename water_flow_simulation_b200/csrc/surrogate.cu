@@ -487,7 +487,7 @@ int launch_gemm_bn(int bn, const __nv_bfloat16* A, int lda, const __nv_bfloat16*
 // the block frees TMEM and returns.
 // ---------------------------------------------------------------------------------------------
 constexpr int kWsThreads = 192;
-constexpr int kWsMaxStages = 8;
+constexpr int kWsMaxStages = 8, kWsShared = 225 * 1024;     // shared memory of a CTA at most
 constexpr uint32_t kWsChBytes = GM * 128;   // channel block: 128 rows x 64 bf16
 
 template <int EPI>
@@ -700,12 +700,12 @@ bool launch_gemm_ws(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int
     const int bv = ws_block_rows(M, N, nsm);
     const int stage = (int)kWsChBytes + bv * 128;
     // as many stages as 225 KB of shared memory hold (row block 224: 5, which measured 1 % above 4)
-    const int stages = (225 * 1024 - 1024) / stage < kWsMaxStages ? (225 * 1024 - 1024) / stage : kWsMaxStages;
+    const int stages = (kWsShared - 1024) / stage < kWsMaxStages ? (kWsShared - 1024) / stage : kWsMaxStages;
     const int smem = stages * stage + 1024;         // > half the SM's shared memory: one CTA per SM
     CUtensorMap ta, tb;
     if (!bf16_tile_map(&ta, A, M, K, lda, bv) || !bf16_tile_map(&tb, B, N, K, ldb, GM)) return false;
     auto kern = k_gemm_ws<EPI>;
-    if (allow_shared(kern, smem) != cudaSuccess) return false;
+    if (allow_shared(kern, kWsShared) != cudaSuccess) return false;
     const long long tiles = (long long)((M + bv - 1) / bv) * ((N + GM - 1) / GM);
     const int grid = (int)(tiles < nsm ? tiles : nsm);
     kern<<<grid, kWsThreads, smem, st>>>(ta, tb, M, N, K, bv, stages, D, ldd, bias, err);
