@@ -14,13 +14,14 @@ import os
 
 from . import _native as nat
 
-# candidates: the split pipeline is the fast family on every lattice measured; the
-# register pipeline is kept as a reference point.  A sixth entry 1 runs the edge and special
-# kernels beside the plain kernel (LBM3D.overlap), ctas_per_sm then bounding the plain kernel.
-SINGLE_FP32 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 4), (3, 4, 2, 0, 0), (0, 2, 4, 0, 0),
-               (3, 4, 4, 0, 0, 1), (3, 4, 4, 0, 2, 1), (3, 2, 4, 0, 2, 1)]
-SINGLE_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 8, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 2), (3, 8, 4, 0, 0),
-               (3, 2, 4, 0, 0, 1), (3, 2, 4, 0, 2, 1), (3, 2, 4, 0, 1, 1)]
+# candidates: the split pipeline is the fast family on every lattice measured; the register pipeline is
+# kept as a reference point.  Shapes of one stream only: a caller's own list may hold six-entry tiles (the edge
+# and special kernels beside the plain one, LBM3D.overlap), but how two streams' kernels share the SMs
+# differs from run to run, so a time measured once does not hold.  Two tunings and 500 steps, ms a step:
+# 36M cells float32, (3, 4, 4, 0, 2, 1) 0.857, 1.047 and 0.861, (3, 4, 2, 0, 0) 0.865, 0.865 and 0.891;
+# 8M cells 16-bit, (3, 2, 4, 0, 2, 1) 0.112, 0.128 and 0.110, (3, 2, 2, 0, 0) 0.113, 0.113 and 0.112.
+SINGLE_FP32 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 4), (3, 4, 2, 0, 0), (0, 2, 4, 0, 0)]
+SINGLE_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 8, 0), (3, 4, 4, 0, 0), (3, 2, 4, 0, 2), (3, 8, 4, 0, 0)]
 BATCH_FP16 = [(3, 2, 4, 0, 0), (3, 2, 2, 0, 0), (3, 2, 4, 8, 0), (3, 2, 4, 0, 2), (3, 2, 1, 0, 0)]
 
 _memo: dict = {}
@@ -99,8 +100,8 @@ def tune_single(L, candidates=None, steps=20, warmup=4, cache_path=None):
 
 
 def tune_batch(batch, candidates=None, steps=20, warmup=4, cache_path=None):
-    """Pick the fastest way to step a BatchRun: one launch per kernel class per step with one of
-    the candidate tiles (its cases' lists stay at 64-cell segments), or the whole 20-step chunk
+    """Pick the fastest way to step a BatchRun: one launch over the lists per step with one of the
+    candidate tiles (its cases' lists stay at 64-cell segments), or the whole 20-step chunk
     in one persistent launch (candidate "persistent").  Each is timed on whole chunks (the last
     step writing the fields), as BatchRun runs them; populations and fields are restored."""
     torch = batch.torch
