@@ -140,10 +140,6 @@ __device__ __forceinline__ long long pull_offset(const PullOffsets& po, bool lid
 // wrote them has ended, and waits for it): the plain kernels issue all of a segment's loads before
 // the first shuffle or conversion waits for one.  The predicated ones leave `v` as it is in the
 // lanes where `on` is false.
-__device__ __forceinline__ void ld_ordered(uint32_t (&v)[1], const void* p)
-{
-    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v[0]) : "l"(p));
-}
 __device__ __forceinline__ void ld_ordered(uint32_t (&v)[2], const void* p)
 {
     asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(p));

@@ -27,11 +27,6 @@
 // with later ones not yet issued (VP = 8: 366 us against 404 on the 36M-cell reach).
 template <int VP> struct HVec;
 template <> struct HVec<4> {
-    static __device__ __forceinline__ void load(uint32_t (&t)[2], const __half* p)
-    {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
-        t[0] = v.x; t[1] = v.y;
-    }
     static __device__ __forceinline__ void store(__half* p, const uint32_t (&t)[2])
     {
         *reinterpret_cast<uint2*>(p) = make_uint2(t[0], t[1]);
@@ -39,22 +34,15 @@ template <> struct HVec<4> {
 };
 // Stores are plain write-back stores: for this kernel they measured 2.7 % faster than
 // streaming (.cs) stores on reach36m, while the float32 kernels keep .cs stores (6 % slower
-// without); .cs, .nc.L1::no_allocate loads were 9-11 % slower than the default read-only ones.
+// without).
 template <> struct HVec<8> {
-    static __device__ __forceinline__ void load(uint32_t (&t)[4], const __half* p)
-    {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
-        t[0] = v.x; t[1] = v.y; t[2] = v.z; t[3] = v.w;
-    }
     static __device__ __forceinline__ void store(__half* p, const uint32_t (&t)[4])
     {
         *reinterpret_cast<uint4*>(p) = make_uint4(t[0], t[1], t[2], t[3]);
     }
 };
 
-// Packed loads of VP cells and of one 4-byte word: read-only path for __half, coherent for hcoh.
-template <int VP>
-__device__ __forceinline__ void hload(uint32_t (&t)[VP / 2], const __half* p) { HVec<VP>::load(t, p); }
+// Coherent packed loads of VP cells and of one 4-byte word (hcoh; __half goes through ld_ordered).
 template <int VP>
 __device__ __forceinline__ void hload(uint32_t (&t)[VP / 2], const hcoh* p)
 {
@@ -66,7 +54,6 @@ __device__ __forceinline__ void hload(uint32_t (&t)[VP / 2], const hcoh* p)
         t[0] = v.x; t[1] = v.y;
     }
 }
-__device__ __forceinline__ uint32_t hword(const __half* p) { return __ldg(reinterpret_cast<const unsigned int*>(p)); }
 __device__ __forceinline__ uint32_t hword(const hcoh* p) { return __ldcg(reinterpret_cast<const unsigned int*>(p)); }
 
 template <int I, int VP, typename T>

@@ -15,17 +15,15 @@
 //   C  bounce-back from solid neighbours, only in lanes whose cells have any;
 //   D  x edges: a direction whose source lies outside [0, nx) keeps the own population.
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-struct PullCtxT {
-    const T* fs;
+struct PullCtx {
+    const float* fs;
     long long S, rowc, own;   // own = rowc + x0c (load start, clamped into the row)
     int x0, x0c, y, z, lane;
 };
-using PullCtx = PullCtxT<float>;
 
-template <int I, int V, typename T>
+template <int I, int V>
 __device__ __forceinline__ void pull_load(float (&t)[Q][V], float (&hv)[Q], uint32_t& rwm, const lbm_lattice& L,
-                                          const PullCtxT<T>& c)
+                                          const PullCtx& c)
 {
     constexpr int CXI = cx(I), CYI = cy(I), CZI = cz(I);
     if constexpr (I == 0) {
@@ -34,7 +32,7 @@ __device__ __forceinline__ void pull_load(float (&t)[Q][V], float (&hv)[Q], uint
         int ys = c.y - CYI, zs = c.z - CZI, di = I;
         if (CZI == -1 && c.z == L.nz - 1) { zs = c.z; di = mirz(I); }   // rigid lid: mirrored population
         const bool rowwall = (ys < 0) || (ys >= L.ny) || (zs < 0);      // warp-uniform
-        const T* row = rowwall ? c.fs + (long long)opp(I) * c.S + c.rowc
+        const float* row = rowwall ? c.fs + (long long)opp(I) * c.S + c.rowc
                                : c.fs + (long long)di * c.S + ((long long)zs * L.ny + ys) * L.pitch;
         ldv<V>(t[I], row + c.x0c);
         if constexpr (CXI == 1) hv[I] = ld1(row + (c.x0c > 0 ? c.x0c - 1 : 0));
@@ -68,9 +66,9 @@ __device__ __forceinline__ void pull_shift(float (&f)[V][Q], float (&t)[Q][V], c
     }
 }
 
-template <int I, int V, typename T>
+template <int I, int V>
 __device__ __forceinline__ void pull_bounce(float (&f)[V][Q], const uint32_t (&fl)[V], uint32_t bb,
-                                            const PullCtxT<T>& c)
+                                            const PullCtx& c)
 {
     if constexpr (I > 0) {
         if (bb & (1u << I)) {
@@ -83,8 +81,8 @@ __device__ __forceinline__ void pull_bounce(float (&f)[V][Q], const uint32_t (&f
     }
 }
 
-template <int I, int V, typename T>
-__device__ __forceinline__ void pull_edge(float (&f)[V][Q], const lbm_lattice& L, const PullCtxT<T>& c)
+template <int I, int V>
+__device__ __forceinline__ void pull_edge(float (&f)[V][Q], const lbm_lattice& L, const PullCtx& c)
 {
     constexpr int CXI = cx(I);
     if constexpr (CXI == 1) {
@@ -98,30 +96,24 @@ __device__ __forceinline__ void pull_edge(float (&f)[V][Q], const lbm_lattice& L
 
 // Rows on the y walls, the bed or the lid: per-direction source rows (phases A and B).
 // Returns the mask of directions whose source row lies outside the domain.
-template <int V, typename T, int... Is>
+template <int V, int... Is>
 __device__ __forceinline__ uint32_t pull_rows(std::integer_sequence<int, Is...>, float (&f)[V][Q],
-                                              const lbm_lattice& L, const PullCtxT<T>& c)
+                                              const lbm_lattice& L, const PullCtx& c)
 {
     float t[Q][V];
     float hv[Q];
     uint32_t rwm = 0;
-    (pull_load<Is, V, T>(t, hv, rwm, L, c), ...);
+    (pull_load<Is, V>(t, hv, rwm, L, c), ...);
     (pull_shift<Is, V>(f, t, hv, rwm, c.lane), ...);
     return rwm;
 }
-template <int V, typename T, int... Is>
-__device__ __forceinline__ void pull_edges(std::integer_sequence<int, Is...>, float (&f)[V][Q], const lbm_lattice& L,
-                                           const PullCtxT<T>& c)
-{
-    (pull_edge<Is, V, T>(f, L, c), ...);                            // phase D only
-}
-template <int V, typename T, int... Is>
+template <int V, int... Is>
 __device__ __forceinline__ void pull_fixups(std::integer_sequence<int, Is...>, float (&f)[V][Q], const lbm_lattice& L,
-                                            const PullCtxT<T>& c, const uint32_t (&fl)[V], uint32_t bb)
+                                            const PullCtx& c, const uint32_t (&fl)[V], uint32_t bb)
 {
-    if (bb) { (pull_bounce<Is, V, T>(f, fl, bb, c), ...); }         // phase C
+    if (bb) { (pull_bounce<Is, V>(f, fl, bb, c), ...); }            // phase C
     const bool edge = (c.x0 == 0) || (c.x0 <= L.nx - 1 && L.nx - 1 < c.x0 + V);
-    if (edge) { (pull_edge<Is, V, T>(f, L, c), ...); }              // phase D
+    if (edge) { (pull_edge<Is, V>(f, L, c), ...); }                 // phase D
 }
 
 // Pull for the segment of an interior row (no y wall or bed involved; `lid`: the row under
