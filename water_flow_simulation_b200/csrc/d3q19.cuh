@@ -41,12 +41,19 @@ __host__ __device__ constexpr double wgt64(int i) {
 // itself, across an x end the cell's own, under the lid the mirrored one, else the neighbour's.
 // The planes' bases and the offsets are uniform, so a lane selects one and adds.  64-bit sums: the
 // opposite direction's plane is S cells away, so own and offset together pass 2^31 on lattices of
-// more than 2^30 cells (16-bit storage of 1.5e9 cells fits one GPU).
-template <int I>
-__host__ __device__ __forceinline__ long long pull_element(long long own, long long plane, int pitch, long long S,
+// more than 2^30 cells (16-bit storage of 1.5e9 cells fits one GPU).  Int = int32_t, for lattices of up
+// to 2^30 cells: 32-bit sums but under the lid, whose mirrored plane may be two away.
+template <int I, typename Int = long long>
+__host__ __device__ __forceinline__ long long pull_element(Int own, Int plane, int pitch, long long S,
                                                            uint32_t fk, bool lid, bool x_first, bool x_last)
 {
     const bool edge = cx(I) == 1 ? x_first : cx(I) == -1 ? x_last : false;
+    if constexpr (sizeof(Int) == 4 && cz(I) != -1) {
+        Int off = -(cz(I) * plane + cy(I) * pitch + cx(I));
+        if (cx(I)) off = edge ? 0 : off;
+        if (I > 0) off = (fk & (1u << I)) ? (opp(I) - I) * (Int)S : off;
+        return I * S + (own + off);
+    }
     long long off = I * S - (cz(I) * plane + (long long)cy(I) * pitch + cx(I));
     if (cz(I) == -1) off = lid ? mirz(I) * S - ((long long)cy(I) * pitch + cx(I)) : off;
     if (cx(I)) off = edge ? I * S : off;

@@ -30,13 +30,13 @@ __device__ __forceinline__ void load_cell(uint16_t& v, const hcoh* p)
     v = __half_as_ushort(__ldcg(reinterpret_cast<const __half*>(p)));
 }
 
-template <typename T, int... Is>
+template <typename T, typename Int, int... Is>
 __device__ __forceinline__ void pull_cell_all(std::integer_sequence<int, Is...>, float (&f)[Q],
-                                              const T* __restrict__ fs, long long own, long long plane, int pitch,
+                                              const T* __restrict__ fs, Int own, Int plane, int pitch,
                                               long long S, uint32_t fk, bool lid, bool x_first, bool x_last)
 {
     typename Stored<T>::type v[Q];
-    (load_cell(v[Is], fs + pull_element<Is>(own, plane, pitch, S, fk, lid, x_first, x_last)), ...);
+    (load_cell(v[Is], fs + pull_element<Is, Int>(own, plane, pitch, S, fk, lid, x_first, x_last)), ...);
     ((f[Is] = Stored<T>::value(v[Is])), ...);
 }
 
@@ -72,8 +72,8 @@ __device__ __forceinline__ bool outlet_across_passes(const lbm_lattice& L, int j
 
 // One warp pass over the cells x = xa + lane of row (y, z) of a special segment
 // (floodsim/lbm3d.py:42-138): `fk` is the lane's flag word (FLAG_SOLID past the pitch), JOIN as in
-// outlet_across_passes.  Called by all lanes of the warp.
-template <int JOIN, bool OUT, bool UCOL, bool AVG, typename T>
+// outlet_across_passes, Int as in pull_element.  Called by all lanes of the warp.
+template <int JOIN, bool OUT, bool UCOL, bool AVG, typename T, typename Int = long long>
 __device__ __forceinline__ void cell_pass(const lbm_lattice& L, const T* __restrict__ fs, T* __restrict__ fd,
                                           float scale, float inv_scale, int xa, int y, int z, int lane, uint32_t fk)
 {
@@ -81,11 +81,11 @@ __device__ __forceinline__ void cell_pass(const lbm_lattice& L, const T* __restr
     const long long S = L.cells;
     const int x = xa + lane;
     const bool active = x < L.pitch, solid = (fk & FLAG_SOLID) != 0;
-    const long long plane = (long long)L.ny * L.pitch, own = z * plane + (long long)y * L.pitch + x;
+    const Int plane = (Int)L.ny * L.pitch, own = z * plane + (Int)y * L.pitch + x;
     float f[Q];
     float r = 1.f, ux = 0.f, uy = 0.f, uz = 0.f;
     if (!solid) {
-        pull_cell_all<T>(QS, f, fs, own, plane, L.pitch, S, fk, z == L.nz - 1, x == 0, x == L.nx - 1);
+        pull_cell_all<T, Int>(QS, f, fs, own, plane, L.pitch, S, fk, z == L.nz - 1, x == 0, x == L.nx - 1);
         float U = 0.f, cf = 0.f;
         if (fk & FLAG_WALLFN) {
             if constexpr (UCOL) U = (fk & FLAG_BEDWALL) ? L.colU[(long long)y * L.pitch + x] : 0.f;
