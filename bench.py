@@ -477,7 +477,7 @@ def run_b200(args, rank, world, local_rank):
     one = counts and main["V"] <= 4 and main["tile"][3] != 8 and not any(main["tile"][4:])
     launches = steps * (1 if one else 3) + (steps // CHUNK) * (4 if one else 2) if counts else steps
     gemm = None
-    if rank == 0 and not args.quick:   # the learned warm start's tensor-core GEMM (bf16, float32 accumulation)
+    if rank == 0 and not args.quick:   # lbm_gemm_bf16 on a product of its own (bf16, float32 accumulation)
         try:
             from water_flow_simulation_b200.surrogate import gemm_throughput
             gemm = gemm_throughput()
@@ -604,8 +604,8 @@ def run_b200(args, rank, world, local_rank):
 
 
 def run_ensemble(args, rank, world, local_rank):
-    """24 seeded boat cases of 2M-20M cells (cases.ensemble_case): the 16-bit batch (one launch per
-    kernel class per step, autotuned tile, 20-step chunks as CUDA graphs) against the plain method
+    """24 seeded boat cases of 2M-20M cells (cases.ensemble_case): the 16-bit batch (one launch
+    over all lists per step, autotuned tile, 20-step chunks as CUDA graphs) against the plain method
     (float32, one case at a time).  cases/hour from each case's own step count to t_total.  With
     N ranks the 24 cases are split over the GPUs by cells x steps (batch.balance), each rank
     batching its own share; the aggregate is all cells over the slowest rank's time."""

@@ -257,8 +257,9 @@ int lbm_fused_step_h(const lbm_lattice *lat, const uint16_t *hs, uint16_t *hd, f
                      const lbm_tile *tile, void *stream);
 
 /* Batched 16-bit solves (no counterpart in the reference, which runs one case at a time):
- * `count` lattices (boat cases of any sizes, one run) advanced by one launch per kernel class
- * per step.  Every table is in device memory:
+ * `count` lattices (boat cases of any sizes, one run) advanced by one launch over all their lists
+ * per step, and one for the outlet rows; a step that writes the fields launches per list.  Every
+ * table is in device memory:
  *   lat          count lattice descriptors (each as for lbm_fused_step_h, with its own work
  *                lists built for cells_per_lane 2 and the same uref mode for all);
  *   pull_offsets count * lbm_batch_pull_offsets_bytes() bytes, filled by lbm_batch_init;
@@ -394,12 +395,14 @@ int lbm_conv3_back(const uint16_t *g, int O, int X, int Y, int Z, const uint16_t
  *   im2col     col[v][t*C + c] = x[tap t of v][c]                (C a multiple of 8)
  *   im2col_t   colT[t*C + c][v] = x[tap t of v][c], zero for v up to Vp (C and Vp multiples of 8)
  *   col2im     dx[v][c] = sum of dcol[u][t*C + c] over the (u, t) that read v   (float)
+ *              (im2col and col2im: the column-matrix form of lbm_conv3_*; the network does not need them)
  *   transpose  out[c][r] = in[r][c] (bf16, R rows -> Rp >= R columns, zero padded)
  *   act_grad   g = dy * (y > 0) (relu) or dy, as bf16; dbias[c] += column sums of g
  *   pool2      2x2x2 average (even grid sizes) and pool2_back its gradient (added to din when
  *              accumulate is set)
  *   up2_add    out = nearest 2x upsampling of coarse + skip, and up2_back the coarse gradient
- *   mse        masked mean-square error of pred[v][0..nout) (row stride Cp): loss += and dpred
+ *   mse        masked mean-square error of pred[v][0..nout) (row stride Cp): loss += (the float32 terms
+ *              summed in float64 in a fixed order, rounded once) and dpred (may be pred itself)
  *   adam       Adam step on float32 weights (bias-corrected, step >= 1), refreshing a bf16 copy */
 int lbm_nn_im2col(const uint16_t *x, int C, int X, int Y, int Z, uint16_t *col, void *stream);
 int lbm_nn_im2col_t(const uint16_t *x, int C, int X, int Y, int Z, int64_t Vp, uint16_t *colT, void *stream);

@@ -4,10 +4,10 @@ Replaces the one-case-at-a-time loop of the reference's boat tests
 (floodsim/boat_tests.py:73-113, Run3D.run_to_end at floodsim/reach3d.py:455-467).
 Every case is a Run3D with 16-bit population storage; the batch steps all of them together
 over the work lists of every case concatenated (entries tagged with their case): by default
-one launch per kernel class per step (lbm_batch_step_h), or, with persistent=True, each
+one launch per step over all lists (lbm_batch_step_h), or, with persistent=True, each
 20-step chunk -- the steps of Run3D.advance between two field outputs -- as ONE persistent
 cooperative launch (lbm_batch_chunk_h: every CTA resident for the chunk, grid barriers
-between the steps; measured 17 % slower on the 24-case ensemble, so not the default; the
+between the steps; measured 24 % slower on the 24-case ensemble, so not the default; the
 autotuner times both); either way the chunk is captured once as a CUDA graph and replayed.
 Per case, as Run3D.advance does: the smoothstep force ramp (a scalar of the case's
 lattice descriptor, in device memory, updated between chunks), the time averages in the
@@ -83,7 +83,7 @@ class BatchRun:
         self.tile = nat.Tile(*tile)
         self.use_graphs = use_graphs
         # persistent: a chunk is ONE cooperative launch of all its steps (lbm_batch_chunk_h), else
-        # one launch per kernel class per step (lbm_batch_step_h); the results are the same bit for bit
+        # one launch over all lists per step (lbm_batch_step_h); the results are the same bit for bit
         self.persistent = bool(persistent)
         self._sync = torch.zeros(4, dtype=torch.int32, device=device if device is not None else "cuda")
         self.tol, self.check_every, self.window = tol, int(check_every), int(window)

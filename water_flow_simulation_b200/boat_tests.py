@@ -10,7 +10,7 @@ our own; the reference's descriptive prose is not carried.  `run_test` has the r
 What changes is how the runs are made.  The reference runs the base and boat cases one
 after another in float32; here, by default, all of them -- one base per distinct level and
 every boat variant -- advance together in one `BatchRun` with 16-bit populations (one
-launch per kernel class per step, 20-step chunks replayed as CUDA graphs), each to the step
+launch over all lists per step, 20-step chunks replayed as CUDA graphs), each to the step
 at which `Run3D.run_to_end` would stop it, and the profiles come from the float64 device
 reductions.  `storage="fp32", batched=False` reproduces the reference's sequence exactly.
 """

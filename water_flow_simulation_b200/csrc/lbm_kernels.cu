@@ -1,22 +1,18 @@
 // lbm_kernels.cu -- sm_100a kernels and C ABI of liblbm_b200.so (declared in include/lbm_b200.h).
 //
-// Hot path: k_fused, one launch per D3Q19 time step.
-//   * Persistent CTAs walk work items (x segment, y row); a CTA owns every z of
-//     its item, so z-column sums (the wall model's depth-mean speed) reduce
-//     inside the CTA, deterministically, with no atomics.
-//   * A warp covers 32*V consecutive x cells of one (y,z) row; each lane owns V
-//     cells and moves them with V-wide (64/128-bit) loads and stores.  A pull
-//     from x-1 / x+1 takes the neighbour lane's element by warp shuffle; only
-//     the segment's first / last lane issues one extra scalar load.
-//   * Walls are a per-cell 19-bit mask in a uint32 flag word (built once):
-//     rows outside the domain (y walls, bed) bounce back warp-uniformly, solid
-//     neighbours per cell with one extra load of the own-row opposite direction.
-//   * Inlet/outlet non-equilibrium extrapolation runs in-thread on the
-//     post-collision registers of x=1 / x=nx-2 (same lane), so the reference's
-//     second kernel disappears.
+// Hot path: k_all_lists (fused_all.cuh), one launch per D3Q19 time step over static lists of row
+// segments: plain interior ones, the x ends' (edge) and those with walls, forcing or hulls (special).  A
+// step that writes the fields, is overlapped or has its grid held down takes a kernel per list instead.
+//   * Walls are a per-cell 19-bit mask in a uint32 flag word (built once, setup.cuh); only special
+//     segments read it.
+//   * Inlet/outlet non-equilibrium extrapolation runs on the post-collision registers of x = 1 and
+//     x = nx-2, so the reference's second kernel disappears; where x = nx-2 and nx-1 fall into
+//     different segments a row pass (k_bc_rows) follows.
 //   * Macroscopic fields are written every step only where the next step's
 //     wall function reads them; the last step of a chunk writes them everywhere,
 //     refreshes the column-mean speed and adds the time averages.
+// k_fused (fused_reg.cuh), k_fused_tma and k_fused_async are the float32 alternatives behind
+// lbm_tile.pipeline: one kernel over all rows, z-column sums inside a CTA.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -517,9 +513,12 @@ bool launch_all_lists(const lbm_lattice& L, const T* fs, T* fd, float scale, con
     const int nspread = F32 && warps > 96LL * sm_count() ? (int)((ends + t.warps - 1) / t.warps) : 0;
     // Programmatic dependent launch on lattices of up to 5M cells: the CTAs become resident as the step
     // before drains and wait there for its end (griddepcontrol), so a step does not pay for a launch and
-    // an empty GPU.  20 steps of 192x50x12 float32 178 -> 144 us, 333x61x17 16-bit 269 -> 241, 577x203x25
-    // 16-bit 1396 -> 1328; but 701x305x37 float32 4195 -> 4223 and 1500x602x40 17.77 -> 17.92 ms (16-bit
-    // 11.00 -> 11.12).  A captured step keeps the full dependency.
+    // an empty GPU.  What it saves is about 2 us a step whatever the size: 20 steps of 192x50x12 float32
+    // 178 -> 144 us, 333x61x17 16-bit 269 -> 241; 2.9M cells float32 1548 -> 1513, 16-bit 1317 -> 1261; 4.3M
+    // 2218 -> 2180 and 1486 -> 1453; 4.7M 2281 -> 2239 and 1549 -> 1513.  Above, the share is small and was
+    // not there in every measurement: 6.2M 3420 -> 3384 and 2087 -> 2049, 7.9M averaged 4199 -> 4158 but
+    // once 4195 -> 4223, 11.9M 5446 -> 5413 and 3676 -> 3645, 23M averaged 10820 -> 10805 and 6857 -> 6852,
+    // 36M within the power cap's spread either way.  A captured step keeps the full dependency.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (L.cells <= kEarlyLaunchCells && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusNone) {

@@ -1,14 +1,14 @@
 // surrogate.cu -- BF16 tensor-core kernels of the learned warm start (sm_100a, tcgen05).
 //
 // The network is a small 3D convolutional encoder-decoder on a coarse copy of the lattice.
-// Every convolution, forward and backward, is a GEMM on 5th-generation tensor cores:
+// Every convolution, forward and backward, is a product on 5th-generation tensor cores:
 //   D[M x N] = A[M x K] * B[N x K]^T      A, B bf16, both K-major; accumulation f32 in TMEM
 // finished by fused epilogues (bias, ReLU, bf16 store).  k_conv_fwd and k_conv_back read the
 // grids in place (no column matrix), k_conv_in that of the first layer (8 channels); the weight gradients
-// go through gather kernels (k_im2col_t, transposes) and three GEMM kernels, chosen per call:
-//   k_gemm_ws    products with >= 1024 rows and >= 128 columns: persistent, warp-specialised,
-//                TMA ring + MMA thread + epilogue warps, accumulator transposed in TMEM;
-//   k_gemm_tma   smaller products: one tile per CTA, TMA ring, MMA thread;
+// go through gather kernels (k_im2col_t, transposes) and lbm_gemm_bf16, whose kernel is chosen per call:
+//   k_gemm_ws    products with >= 1024 rows and >= 128 columns (none of the network's): persistent,
+//                warp-specialised, TMA ring + MMA thread + epilogue warps, accumulator transposed in TMEM;
+//   k_gemm_tma   smaller products (the weight gradients): one tile per CTA, TMA ring, MMA warp;
 //   k_gemm_bf16  when no tensor map can be made: the register-staged kernel described here.
 //
 // k_gemm_bf16 tile: one CTA computes 128 rows x BN columns.  Per 64-wide K step, the 4 warps copy
@@ -463,8 +463,8 @@ int launch_gemm_bn(int bn, const __nv_bfloat16* A, int lda, const __nv_bfloat16*
 }
 
 // ---------------------------------------------------------------------------------------------
-// Persistent warp-specialised GEMM for products with many rows and N >= 128 (the convolutions'
-// voxels x channels).  The accumulator is held transposed: tcgen05.mma with M = 128 takes a
+// Persistent warp-specialised GEMM for products with many rows and N >= 128 (a caller's; the network's own
+// have at most 128 rows, and its convolutions read the grids in place).  The accumulator is held transposed: tcgen05.mma with M = 128 takes a
 // 128-row block of B (output channels n0..n0+127) as its A operand and a BV-row block of A
 // (voxels m0..m0+BV-1, BV = 128..256) as its B operand, so TMEM lane l holds channel n0 + l and
 // column j voxel m0 + j.  The epilogue thread of lane l then writes 32 voxels of one channel,
@@ -720,8 +720,9 @@ int launch_gemm_any(int bn, const __nv_bfloat16* A, int lda, const __nv_bfloat16
     int status = LBM_OK;
     // D += products with a long K and few tiles (the weight gradients: K is the voxels): narrow tiles,
     // for as many CTAs as there are, and a ring deep enough that the one chain of MMAs never waits
-    // for a load.  64 x 1728 weights over 12,288 voxels: 54 CTAs instead of 7, 88 -> 43 us a layer.  Splitting
-    // K would be faster still, but moves the sums by more than 2e-5.
+    // for a load.  64 x 1728 weights over 12,288 voxels: 54 CTAs instead of 7, 64 us (the six layers of a
+    // training step 88 -> 43 us on average).  Splitting K would be faster still, but moves the sums by more
+    // than 2e-5.
     if constexpr (EPI == EPI_F32_ADD) {
         const long long wide = (long long)((M + GM - 1) / GM) * ((N + bn - 1) / bn);
         if (wide * 2 <= sm_count() && K >= 4 * GK &&
@@ -811,7 +812,7 @@ __device__ __forceinline__ void conv_store(uint32_t lane_addr, long long v, int 
 
 // Forward: D[v][n] = epilogue(sum_t sum_c x[v + off_t][c] W[n][t*C + c] + bias[n]), C a multiple of
 // 64.  One box x BN channels per CTA (two CTAs per SM, so one's epilogue runs beside the other's
-// loads), one loading thread, one MMA thread, a ring of S stages; waits bounded as in k_gemm_tma.
+// loads), one loading warp, one MMA warp, a ring of S stages; waits bounded as in k_gemm_tma.
 template <int BN, int EPI, int S>
 __global__ void __launch_bounds__(128, 2) k_conv_fwd(const __grid_constant__ CUtensorMap tmX,
                                                      const __grid_constant__ CUtensorMap tmW, const ConvTiles g, int C,

@@ -3,8 +3,9 @@
 Same constructor, same public arrays (``f, f2, rho, ux, uy, uz, Fx, Fy, Fz, uin,
 uref, cfw, solid``), same ``step(n)``, ``set_force``, ``shape3`` and
 ``memory_mb``, same ``TypeError`` on a force/inlet/uref array of the wrong dtype
-or size.  Arrays are torch CUDA tensors.  Every step is one launch of the fused
-kernel of liblbm_b200.so (``lbm_fused_step``); there is no CPU path.
+or size.  Arrays are torch CUDA tensors.  Every step is one call of
+liblbm_b200.so (``lbm_fused_step``): one launch over the lattice's work lists, or,
+when it writes the fields, one per list; there is no CPU path.
 
 Additions, all optional and off by default:
 
@@ -410,7 +411,7 @@ class LBM3D:
 
     # ------------------------------------------------------------------ stepping
     def step(self, n=1, accumulate=False):
-        """Advance n time steps (floodsim/lbm3d.py:390-412): one fused launch each."""
+        """Advance n time steps (floodsim/lbm3d.py:390-412): one library call each."""
         if self._bad:
             name, (dt, size) = next(iter(self._bad.items()))
             raise TypeError(f"LBM3D: force/inlet arrays must be float32 of the correct size (got {dt}, {size})")

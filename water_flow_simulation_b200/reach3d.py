@@ -12,8 +12,8 @@ names, arguments and results:
   reference's (tests/test_reach_builder.py);
 * ``Run3D`` (reach3d.py:378-497) -- the time loop on ``LBM3D``: 20-step chunks,
   smoothstep force ramp, column-mean wall-model speed and time averages, here all
-  done inside the fused kernel (a scalar force scale, the kernel's column-mean
-  refresh and its accumulation epilogue) instead of by separate array passes;
+  done inside the library's step (a scalar force scale, the column-mean refresh and the
+  accumulation epilogue of the step that writes the fields) instead of by separate array passes;
 * ``profiles``, ``compare`` (reach3d.py:545-618) -- water level, discharge, bed
   shear, momentum flux and the boat-versus-base comparison.
 

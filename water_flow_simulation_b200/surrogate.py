@@ -255,8 +255,9 @@ class SurrogateNet:
 
 
 def gemm_throughput(M=32768, N=128, K=3456, reps=20, device=None):
-    """TFLOP/s of lbm_gemm_bf16 on an M x N x K product (the forward GEMM of the 128 -> 128
-    convolution on M coarse voxels), CUDA events around `reps` launches after a warm-up."""
+    """TFLOP/s of lbm_gemm_bf16 on an M x N x K product of its own (the size of a 128 -> 128 convolution
+    on M coarse voxels written as a matrix product; the network's convolutions read the grids in place,
+    lbm_conv3_bf16), CUDA events around `reps` launches after a warm-up."""
     torch = nat.require_cuda()
     lib = nat.load()
     dev = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
