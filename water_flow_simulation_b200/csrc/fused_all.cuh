@@ -30,6 +30,8 @@ __global__ void __launch_bounds__(128, std::is_same<T, float>::value ? 4 : 5)
 {
     constexpr int SEG = 32 * CPL, G = SEG / 4 < 32 ? SEG / 4 : 32;
     constexpr bool F32 = std::is_same<T, float>::value;
+    // steps launched early are those of small lattices (kEarlyLaunchCells): 32-bit indexes (pull_element)
+    using Int = std::conditional_t<EARLY, int, long long>;
     const int lane = threadIdx.x & 31, nseg = (L.pitch + SEG - 1) / SEG;
     const float inv_scale = 1.0f / scale;
     if constexpr (EARLY) {
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(128, std::is_same<T, float>::value ? 4 : 5)
         decode_row(__ldg(L.rows_special + t / CPL), nseg, L.ny, seg, y, z);
         const int xa = seg * SEG + t % CPL * 32;
         if (xa < L.pitch)
-            cell_pass<SEG < 128 ? SEG : 128, false, UCOL, false, T>(L, fs, fd, scale, inv_scale, xa, y, z, lane,
+            cell_pass<SEG < 128 ? SEG : 128, false, UCOL, false, T, Int>(L, fs, fd, scale, inv_scale, xa, y, z, lane,
                                                                    pass_flags(L, xa + lane, y, z));
         return;
     }

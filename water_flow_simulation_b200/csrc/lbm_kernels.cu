@@ -494,6 +494,7 @@ int launch_cells(const lbm_lattice& L, const T* fs, T* fd, float scale, const lb
 }
 
 constexpr long long kEarlyLaunchCells = 5'000'000;         // launch_all_lists
+static_assert(kEarlyLaunchCells <= 1LL << 30, "k_all_lists<EARLY> takes 32-bit indexes");
 
 // The three lists in one launch (k_all_lists): whenever the call leaves the grid and the streams to
 // the launcher.  false: one launch per list.  With float32 storage and more than 96 warps per SM (six
