@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(128, std::is_same<T, float>::value ? 4 : 5)
         const int xa = seg * SEG + t % CPL * 32;
         if (xa < L.pitch)
             cell_pass<SEG < 128 ? SEG : 128, false, UCOL, false, T, Int>(L, fs, fd, scale, inv_scale, xa, y, z, lane,
-                                                                   pass_flags(L, xa + lane, y, z));
+                                                                         pass_flags(L, xa + lane, y, z));
         return;
     }
     t -= ncells;
